@@ -12,7 +12,8 @@ LDLIBS    := -lpthread -ldl -lrt
 
 TYPES := i8:int8_t u8:uint8_t i32:int32_t u32:uint32_t i64:int64_t u64:uint64_t f16:__half f32:float f64:double bf16:__nv_bfloat16
 NVLS_TYPES := f16 f32 bf16
-TYPE_OBJS := $(foreach t,$(TYPES),$(OBJ)/inst_$(word 1,$(subst :, ,$(t))).o) $(foreach t,$(TYPES),$(OBJ)/batch_$(word 1,$(subst :, ,$(t))).o)
+TYPE_OBJS := $(foreach t,$(TYPES),$(OBJ)/inst_$(word 1,$(subst :, ,$(t))).o) $(foreach t,$(TYPES),$(OBJ)/batch_$(word 1,$(subst :, ,$(t))).o) \
+             $(foreach t,$(TYPES),$(OBJ)/one_gpu_$(word 1,$(subst :, ,$(t))).o)
 
 HOST_SRCS := csrc/common/value.cc csrc/common/log.cc csrc/ipc/uds.cc csrc/device/host_backend.cc \
              csrc/daemon/config.cc csrc/daemon/transport.cc csrc/daemon/planner.cc csrc/daemon/qos.cc csrc/daemon/trace.cc \
@@ -53,6 +54,9 @@ $(OBJ)/inst_$(1).o: csrc/kernels/inst_dtype.cu $(HDRS)
 $(OBJ)/batch_$(1).o: csrc/kernels/inst_batch.cu $(HDRS)
 	@mkdir -p $$(dir $$@)
 	$(NVCC) $(NVCCFLAGS) -DMCCS_T=$(2) -DMCCS_TNAME=$(1) $(if $(filter $(1),$(NVLS_TYPES)),-DMCCS_NVLS=1) -c $$< -o $$@ 2> $$@.log || (cat $$@.log; false)
+$(OBJ)/one_gpu_$(1).o: csrc/kernels/inst_one_gpu.cu $(HDRS)
+	@mkdir -p $$(dir $$@)
+	$(NVCC) $(NVCCFLAGS) -DMCCS_T=$(2) -DMCCS_TNAME=$(1) -c $$< -o $$@ 2> $$@.log || (cat $$@.log; false)
 endef
 $(foreach t,$(TYPES),$(eval $(call TYPE_RULE,$(word 1,$(subst :, ,$(t))),$(word 2,$(subst :, ,$(t))))))
 
@@ -112,8 +116,13 @@ build/sim/kernel_sim_test: csrc/tests/kernel_sim_test.cc $(wildcard csrc/tests/s
 	@mkdir -p build/sim
 	$(SAN_CXX) -std=c++17 -O1 -g -Wall -Wno-unknown-pragmas -Wno-unused-parameter -pthread -I/usr/local/cuda/include -o $@ csrc/tests/kernel_sim_test.cc
 
-simtest: build/sim/kernel_sim_test
+build/sim/one_gpu_sim_test: csrc/tests/one_gpu_sim_test.cc $(wildcard csrc/tests/sim/*.h) $(HDRS)
+	@mkdir -p build/sim
+	$(SAN_CXX) -std=c++17 -O1 -g -Wall -Wno-unknown-pragmas -Wno-unused-parameter -pthread -I/usr/local/cuda/include -o $@ csrc/tests/one_gpu_sim_test.cc
+
+simtest: build/sim/kernel_sim_test build/sim/one_gpu_sim_test
 	build/sim/kernel_sim_test
+	build/sim/one_gpu_sim_test
 
 tsan: build/san/stress_tsan
 	TSAN_OPTIONS="halt_on_error=0 second_deadlock_stack=1 suppressions=csrc/tests/tsan.supp" build/san/stress_tsan 40

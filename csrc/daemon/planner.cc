@@ -164,6 +164,9 @@ std::string Planner::infeasible(int variant, const PlanInput& in) {
     case kRsDirect: case kRsNvls:
       if (in.kind != kReduceScatter) return "reduce-scatter variant requested for another collective";
       break;
+    case kOneGpu:
+      if (in.nranks > 1 && !in.emulated) return "the ranks sit on different devices";
+      break;
     default:
       return "unknown variant";
   }
@@ -200,6 +203,9 @@ Plan Planner::plan(const PlanInput& in) const {
   // Candidate order: the requested variant, the table's pick, then safe fall-backs.
   std::vector<int> candidates;
   if (in.requested_variant > 0) candidates.push_back(in.requested_variant);
+  // Ranks that share a GPU need no rank-to-rank protocol and no tuned grid. (The tables are
+  // measured with one GPU per rank; an explicit request still gets the kernel it names.)
+  if (in.emulated && !(is_ar && in.fusable)) candidates.push_back(kOneGpu);
   if (e) candidates.push_back(e->variant);
   if (in.nranks == 1) candidates.push_back(kLocalCopy);
   if (is_rs) {
@@ -233,6 +239,7 @@ Plan Planner::plan(const PlanInput& in) const {
   // The hybrid kernel runs two data paths side by side: the peer-copy part wants as many
   // CTAs as the plain two-shot exchange on top of the few that feed the switch.
   if (chosen == kArHybrid && !(e && e->variant == chosen)) ctas = p.bytes <= 4 * MB_ ? 24 : 72;
+  if (chosen == kOneGpu) ctas = kMaxCtas;   // follows the message unless a quota bounds it
   if (variant_is_ring(chosen)) {
     ctas = in.ring_channels > 0 ? in.ring_channels : 1;
     // Small messages do not fill several channels: drop to one, then shrink the CTA,
@@ -246,6 +253,7 @@ Plan Planner::plan(const PlanInput& in) const {
   if (variant_is_ring(chosen) && ctas > kMaxRingChannels) ctas = kMaxRingChannels;
   if (ctas > kMaxCtas) ctas = kMaxCtas;
   if (ctas < 1) ctas = 1;
+  p.bounded = in.requested_ctas > 0 || in.cta_cap > 0;
   // Never launch more CTAs than there are 16-byte packs per rank to move.
   const uint64_t packs = std::max<uint64_t>(1, p.bytes / 16 / (uint64_t)threads / (uint64_t)in.nranks);
   if (!variant_is_ring(chosen) && (uint64_t)ctas > packs) ctas = (int)packs;

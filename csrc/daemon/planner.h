@@ -43,6 +43,7 @@ struct PlanInput {
   bool host_staged = false;     // transport forces FIFO rings through pinned host memory
   uint32_t carried_variants = ~0u;  // bit v: every connection of the communicator can carry variant v (ConnectionTable)
   bool emulated = false;        // all ranks on one device (single cooperative launch)
+  bool fusable = false;         // several queued all-reduces may share a launch (keeps the variants that have a fused form)
   int requested_variant = kAuto;  // from the caller or an override
   int requested_ctas = 0;         // from an override ("channel count"), 0 = table
   int cta_cap = 0;                // QoS quota, 0 = none
@@ -54,6 +55,7 @@ struct Plan {
   int variant = kAuto;
   LaunchDims dims{1, 512};
   uint64_t bytes = 0;           // message size used for the table lookup and accounting
+  bool bounded = false;         // dims.ctas is a limit set by a quota or an operator, not just the planner's choice
   bool needs_mc_send = false;   // multicast mapping of the send allocations required
   bool needs_mc_recv = false;
   int status = 0;               // proto::Status; non-zero: cannot run

@@ -292,6 +292,7 @@ bool ProxyEngine::plan_slot(Communicator& c, CollSlot& s, uint64_t seq) {
   in.emulated = c.emulated;
   in.host_staged = c.host_staged;
   in.fifo_slot_bytes = c.fifo_slot_bytes;
+  in.fusable = daemon_->config().fuse_allreduce > 1 || daemon_->config().single_through_fused;
   // Every block boundary the kernels compute from the count must be aligned as well.
   uint64_t bits = o0.kind == kAllGather ? o0.count : o0.kind == kReduceScatter ? o0.count * (uint64_t)dtype_size(o0.dtype) : 0;
   bool same_send_off = true, same_recv_off = true, all_vmm = !host_backend || be->nvls_supported();   // the host backend's emulated multicast binds any of its allocations
@@ -359,7 +360,7 @@ bool ProxyEngine::plan_slot(Communicator& c, CollSlot& s, uint64_t seq) {
     if (fifo_channels < 1) return fail(proto::kErrUnsupported);
     plan.dims.ctas = std::min(plan.dims.ctas, fifo_channels);
   }
-  if (c.emulated && !host_backend) {
+  if (c.emulated && !host_backend && variant_waits(plan.variant)) {
     int fit = be->max_group_ctas(plan.variant, in.dtype, in.op, plan.dims.threads, c.nranks);
     if (fit < 1) return fail(proto::kErrUnsupported);
     plan.dims.ctas = std::min(plan.dims.ctas, fit);
@@ -585,7 +586,8 @@ bool ProxyEngine::admit_slice(Communicator& c, CollSlot& s, int slice) {
   if (s.admitted_slices.load(std::memory_order_acquire) > slice) return true;
   const uint64_t bytes = s.batch_len > 1 ? s.batch_bytes : s.nslices == 1 ? s.plan.bytes : s.plan.bytes / (uint64_t)s.nslices;
   // CTAs per GPU: one launch per rank and GPU, or every rank's CTAs on the one GPU.
-  const int ctas = s.plan.dims.ctas * (c.emulated ? c.nranks : 1);
+  // None where the kernel's CTAs do not wait for one another: such a launch can always run.
+  const int ctas = !variant_waits(s.plan.variant) ? 0 : s.plan.dims.ctas * (c.emulated ? c.nranks : 1);
   // A request that was told to wait is not put to the arbiter again (a lock shared by the
   // proxies of all GPUs) until the arbiter's state moved, or a short time passed for the
   // reasons that follow the clock: 20 us for a closed window, 200 us otherwise (a competitor
@@ -650,6 +652,8 @@ void ProxyEngine::fill_args(Communicator& c, CollSlot& s, int rank, int slice, C
     a.unroll_hint = daemon_->config().nvls_unroll;
   } else if (s.plan.variant == kAgPull || s.plan.variant == kAgPush || s.plan.variant == kArTwoShot) {
     a.unroll_hint = daemon_->config().pack_bytes;
+  } else if (s.plan.variant == kOneGpu) {
+    a.unroll_hint = s.plan.bounded ? s.plan.dims.ctas * c.nranks : 0;
   }
   a.fifo_slot_bytes = c.fifo_slot_bytes;
   memcpy(a.ring, s.ring, sizeof a.ring);

@@ -632,7 +632,7 @@ class CudaBackend : public Backend {
 
   int launch(int dev, int kind, const CollArgs& a, LaunchDims dims, void* stream) override {
     (void)dev;
-    cudaError_t e = launch_collective(kind, a, dims, stream);
+    cudaError_t e = a.variant == kOneGpu ? launch_one_gpu(kind, a, a.unroll_hint, true, stream) : launch_collective(kind, a, dims, stream);
     if (e != cudaSuccess) {
       LOG_ERROR("launch %s failed: %s", variant_name(a.variant), cudaGetErrorString(e));
       cudaGetLastError();

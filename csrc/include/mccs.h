@@ -94,7 +94,8 @@ typedef enum {
   mccsAlgoAgNvls = 8, mccsAlgoAgRing = 9, mccsAlgoLocalCopy = 10,
   mccsAlgoArHybrid = 11,  /* part through the switch, part by peer copies, in one kernel */
   mccsAlgoRsDirect = 12,  /* reduce-scatter by peer loads */
-  mccsAlgoRsNvls = 13     /* reduce-scatter in the switch */
+  mccsAlgoRsNvls = 13,    /* reduce-scatter in the switch */
+  mccsAlgoOneGpu = 14     /* ranks that share a GPU: all inputs to all outputs in one pass, any collective */
 } mccsAlgo_t;
 
 /* Connects to the daemon. Optional: every other call connects on first use with

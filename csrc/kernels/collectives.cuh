@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(kMaxThreads) local_copy_kernel(const __grid_co
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = done + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < bytes; i += stride) out[i] = in[i];
   }
-  finish(a, rank);
+  if (a.pad[rank] != nullptr) finish(a, rank);   // no completion word for callers without a communicator
 }
 
 #endif  // MCCS_UNTYPED_KERNELS

@@ -137,6 +137,53 @@ template <> __device__ __forceinline__ void st_data<16>(void* p, Raw<16> v) {
                "r"(v.y), "r"(v.z), "r"(v.w));
 }
 
+// Loads and stores of this GPU's own memory by kernels that no other GPU takes part in: weak
+// accesses, cached in L1 (visible across kernels by stream order).
+template <int BYTES> __device__ __forceinline__ Raw<BYTES> ld_local(const void* p);
+template <int BYTES> __device__ __forceinline__ void st_local(void* p, Raw<BYTES> v);
+template <> __device__ __forceinline__ Raw<1> ld_local<1>(const void* p) {
+  uint32_t t;
+  asm volatile("ld.global.u8 %0, [%1];" : "=r"(t) : "l"(p));
+  Raw<1> r; r.x = (uint8_t)t; return r;
+}
+template <> __device__ __forceinline__ Raw<2> ld_local<2>(const void* p) {
+  Raw<2> r;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(r.x) : "l"(p));
+  return r;
+}
+template <> __device__ __forceinline__ Raw<4> ld_local<4>(const void* p) {
+  Raw<4> r;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(r.x) : "l"(p));
+  return r;
+}
+template <> __device__ __forceinline__ Raw<8> ld_local<8>(const void* p) {
+  Raw<8> r;
+  asm volatile("ld.global.u64 %0, [%1];" : "=l"(r.x) : "l"(p));
+  return r;
+}
+template <> __device__ __forceinline__ Raw<16> ld_local<16>(const void* p) {
+  Raw<16> r;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+template <> __device__ __forceinline__ void st_local<1>(void* p, Raw<1> v) {
+  asm volatile("st.global.u8 [%0], %1;" ::"l"(p), "r"((uint32_t)v.x));
+}
+template <> __device__ __forceinline__ void st_local<2>(void* p, Raw<2> v) {
+  asm volatile("st.global.u16 [%0], %1;" ::"l"(p), "h"(v.x));
+}
+template <> __device__ __forceinline__ void st_local<4>(void* p, Raw<4> v) {
+  asm volatile("st.global.u32 [%0], %1;" ::"l"(p), "r"(v.x));
+}
+template <> __device__ __forceinline__ void st_local<8>(void* p, Raw<8> v) {
+  asm volatile("st.global.u64 [%0], %1;" ::"l"(p), "l"(v.x));
+}
+template <> __device__ __forceinline__ void st_local<16>(void* p, Raw<16> v) {
+  asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
+}
+// The low word of (hi:lo) >> bits, 0 <= bits < 32.
+__device__ __forceinline__ uint32_t funnel_right(uint32_t lo, uint32_t hi, uint32_t bits) { return __funnelshift_r(lo, hi, bits); }
+
 // ----------------------------------------------------------------------------
 // NVLS: one instruction addressed at a multicast mapping is executed by the
 // NVSwitch against every GPU bound to it (sum in the switch / replicate a store).

@@ -55,7 +55,8 @@ enum Variant : int32_t {
   kArHybrid = 11,    // head of the buffer through the switch (multimem), rest by peer loads/stores, in one kernel
   kRsDirect = 12,    // reduce-scatter: every rank loads its block from all peers and reduces it
   kRsNvls = 13,      // reduce-scatter: multimem.ld_reduce of the own block
-  kNumVariants = 14
+  kOneGpu = 14,      // every rank on one GPU: all ranks' inputs to all ranks' outputs in one pass, no rank-to-rank protocol
+  kNumVariants = 15
 };
 
 // Error codes written by kernels into the per-rank status word.
@@ -121,7 +122,8 @@ struct CollArgs {
   int32_t trace;           // 1: record globaltimer start/end into the status block
   int32_t unroll_hint;     // ar_hybrid: low 16 bits = share of the message for the multimem part (1/1000), high 16 bits = its CTAs;
                            // the NVLS all-reduce kernels: in-switch loads in flight per thread (8, or 4 for any other value);
-                           // all-gather pull/push: 32 = 256-bit loads and stores where buffers and size allow
+                           // all-gather pull/push: 32 = 256-bit loads and stores where buffers and size allow;
+                           // kOneGpu: most CTAs of the whole grid (0 = the grid follows the message)
   // --- buffers (unicast addresses valid on every GPU of the communicator) -----
   const void* send[kMaxRanks];
   void* recv[kMaxRanks];
@@ -168,6 +170,28 @@ struct BatchArgs {
   void* mc_recv[kMaxBatch];
 };
 
+// Launch shape of the one-GPU kernels: at most kGroupThreads threads per CTA, and packs per
+// thread and tile: of a reduction over up to four ranks (one beyond), of a gather for up to four
+// ranks and for more.
+constexpr int kGroupThreads = 256;
+constexpr int kReduceUnrollFew = 2;
+constexpr int kGatherUnrollFew = 4;
+constexpr int kGatherUnrollMany = 2;
+// One launch that carries every rank of a communicator whose ranks share a GPU (kOneGpu).
+struct OneGpuArgs {
+  const void* send[kMaxRanks];
+  void* recv[kMaxRanks];
+  uint64_t count;            // as CollArgs::count
+  int32_t nranks;
+  int32_t kind;              // CollKind
+  int32_t op;                // RedOp
+  int32_t trace;
+  float scale;
+  uint32_t* counter;         // finished CTAs, wraps to zero at the grid size; null = no completion word
+  uint64_t seq;
+  StatusBlock* status[kMaxRanks];
+};
+
 struct LaunchDims {
   int32_t ctas;      // grid.x (per rank)
   int32_t threads;   // block.x
@@ -199,11 +223,14 @@ inline const char* variant_name(int v) {
     case kArHybrid: return "ar_hybrid";
     case kRsDirect: return "rs_direct";
     case kRsNvls: return "rs_nvls";
+    case kOneGpu: return "one_gpu";
   }
   return "?";
 }
 
 inline bool variant_is_nvls(int v) { return v == kArNvlsOne || v == kArNvlsTwo || v == kAgNvls || v == kArHybrid || v == kRsNvls; }
+// Kernels whose CTAs never wait for one another: nothing has to be resident together.
+inline bool variant_waits(int v) { return v != kLocalCopy && v != kOneGpu; }
 inline bool variant_is_ring(int v) { return v == kArRing || v == kAgRing; }
 
 // Number of ring steps one channel consumes for a collective. Every rank and every

@@ -1,6 +1,7 @@
 #include "launch.h"
 
 #include <stdio.h>
+#include <string.h>
 
 extern "C" {
 const void* mccs_kfn_i8(int, int);
@@ -14,6 +15,17 @@ const void* mccs_kfn_f32(int, int);
 const void* mccs_kfn_f64(int, int);
 const void* mccs_kfn_bf16(int, int);
 const void* mccs_kfn_untyped(int);
+const void* mccs_kfn_one_gpu_i8(int, int, int);
+const void* mccs_kfn_one_gpu_u8(int, int, int);
+const void* mccs_kfn_one_gpu_i32(int, int, int);
+const void* mccs_kfn_one_gpu_u32(int, int, int);
+const void* mccs_kfn_one_gpu_i64(int, int, int);
+const void* mccs_kfn_one_gpu_u64(int, int, int);
+const void* mccs_kfn_one_gpu_f16(int, int, int);
+const void* mccs_kfn_one_gpu_f32(int, int, int);
+const void* mccs_kfn_one_gpu_f64(int, int, int);
+const void* mccs_kfn_one_gpu_bf16(int, int, int);
+const void* mccs_kfn_group_gather(int, int);
 const void* mccs_kfn_batch_i8(int, int);
 const void* mccs_kfn_batch_u8(int, int);
 const void* mccs_kfn_batch_i32(int, int);
@@ -31,6 +43,7 @@ namespace mccs {
 const void* batch_kernel_function(int variant, int dtype, int op);
 
 const void* kernel_function(int variant, int dtype, int op) {
+  if (variant == kOneGpu) return one_gpu_function(kAllReduce, dtype, op, 2, false);   // every type and operator has all forms
   if (variant == kArHybrid || variant == kRsDirect || variant == kRsNvls)
     return batch_kernel_function(variant, dtype, op);   // live with the newer kernels
   switch (variant) {
@@ -65,6 +78,23 @@ const void* batch_kernel_function(int variant, int dtype, int op) {
     case kFloat32: return mccs_kfn_batch_f32(variant, op);
     case kFloat64: return mccs_kfn_batch_f64(variant, op);
     case kBfloat16: return mccs_kfn_batch_bf16(variant, op);
+  }
+  return nullptr;
+}
+
+const void* one_gpu_function(int kind, int dtype, int op, int nranks, bool ragged) {
+  if (kind == kAllGather) return mccs_kfn_group_gather(nranks, ragged);
+  switch (dtype) {
+    case kInt8: return mccs_kfn_one_gpu_i8(nranks, op, ragged);
+    case kUint8: return mccs_kfn_one_gpu_u8(nranks, op, ragged);
+    case kInt32: return mccs_kfn_one_gpu_i32(nranks, op, ragged);
+    case kUint32: return mccs_kfn_one_gpu_u32(nranks, op, ragged);
+    case kInt64: return mccs_kfn_one_gpu_i64(nranks, op, ragged);
+    case kUint64: return mccs_kfn_one_gpu_u64(nranks, op, ragged);
+    case kFloat16: return mccs_kfn_one_gpu_f16(nranks, op, ragged);
+    case kFloat32: return mccs_kfn_one_gpu_f32(nranks, op, ragged);
+    case kFloat64: return mccs_kfn_one_gpu_f64(nranks, op, ragged);
+    case kBfloat16: return mccs_kfn_one_gpu_bf16(nranks, op, ragged);
   }
   return nullptr;
 }
@@ -105,6 +135,57 @@ int max_cooperative_ctas(int variant, int dtype, int op, int threads, int nranks
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0) != cudaSuccess) return 0;
   return sms * per_sm / nranks;
+}
+
+cudaError_t launch_one_gpu(int kind, const CollArgs& args, int max_ctas, bool completion, void* stream) {
+  const int n = args.nranks;
+  if (n < 2 || n > kMaxRanks) return cudaErrorInvalidValue;
+  const uint64_t bytes = args.count * (uint64_t)(kind == kAllGather ? 1 : dtype_size(args.dtype));   // one rank's part, or one block
+  OneGpuArgs a;
+  memset(&a, 0, sizeof a);
+  uint64_t bits = kind == kAllReduce ? 0 : bytes;   // blocks start at multiples of their size
+  for (int r = 0; r < n; r++) {
+    a.send[r] = args.send[r];
+    a.recv[r] = args.recv[r];
+    a.status[r] = args.status[r];
+    bits |= (uint64_t)args.send[r] | (uint64_t)args.recv[r];
+  }
+  const bool ragged = (bits & 15u) != 0;
+  const void* fn = one_gpu_function(kind, args.dtype, args.op, n, ragged);
+  if (!fn) return cudaErrorInvalidDeviceFunction;
+  a.count = args.count;
+  a.nranks = n;
+  a.kind = kind;
+  a.op = args.op;
+  a.trace = args.trace;
+  a.scale = args.scale;
+  a.seq = args.seq;
+  a.counter = completion ? &args.pad[0]->pad_[kPadCtaCounter] : nullptr;
+  const uint64_t groups = kind == kAllReduce ? 1 : (uint64_t)n;
+  const uint64_t packs = (bytes + 15) / 16;
+  const uint64_t unroll = ragged ? 1
+                          : kind == kAllGather ? (n <= 4 ? kGatherUnrollFew : kGatherUnrollMany)
+                                               : (n <= 4 ? kReduceUnrollFew : 1);
+  // 128 threads measured as fast as or faster than 256, as long as a CTA moves 16 KiB: the GPU
+  // starts one CTA in about 2.7 ns, so smaller ones cannot keep up with the memory. The reduction
+  // over more than four ranks needs the larger CTA for large messages (eight ranks, 200 MiB
+  // blocks scattered: 273 us against 352 us) but not for a few waves, where what counts is how
+  // evenly the last CTAs end. The shortest messages are spread until every SM has a CTA.
+  const uint64_t buffers = (kind == kAllGather ? 1 : (uint64_t)n) + (kind == kReduceScatter ? 1 : (uint64_t)n);
+  uint64_t threads = 128;
+  if (threads * unroll * 16 * buffers < 16384 || (kind != kAllGather && n > 4 && packs * groups >= 16ull * kMaxCtas * kGroupThreads * unroll))
+    threads = kGroupThreads;
+  while (threads > 32 && packs * groups < (uint64_t)kMaxCtas * threads * unroll) threads /= 2;
+  uint64_t ctas = (packs + threads * unroll - 1) / (threads * unroll);
+  if (max_ctas > 0 && ctas * groups * threads > (uint64_t)max_ctas * 512) {
+    // A bounded grid (a tenant's share of the SMs, counted in CTAs of 512 threads) loops over the tiles.
+    threads = kGroupThreads;
+    ctas = ((uint64_t)max_ctas * 512 / threads + groups - 1) / groups;
+  }
+  if (ctas < 1) ctas = 1;
+  if (ctas > 0x7fffffffull) ctas = 0x7fffffffull;
+  void* params[] = {(void*)&a};
+  return cudaLaunchKernel(fn, dim3((unsigned)ctas, (unsigned)groups, 1u), dim3((unsigned)threads, 1u, 1u), params, 0, (cudaStream_t)stream);
 }
 
 cudaError_t launch_collective(int kind, const CollArgs& args, LaunchDims dims, void* stream) {

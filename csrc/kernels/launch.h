@@ -15,6 +15,14 @@ cudaError_t launch_collective(int kind, const CollArgs& args, LaunchDims dims, v
 // Largest CTA count per rank that keeps an emulated (cooperative) launch resident.
 int max_cooperative_ctas(int variant, int dtype, int op, int threads, int nranks);
 
+// Every rank of a communicator that shares one GPU, in one launch without rank-to-rank protocol
+// (one_gpu.cuh): `args` as for an emulated launch_collective; `completion`: publish args.seq in
+// the status blocks; `max_ctas` > 0 bounds the grid (in CTAs of 512 threads), otherwise it follows
+// the message.
+cudaError_t launch_one_gpu(int kind, const CollArgs& args, int max_ctas, bool completion, void* stream);
+// The kernel such a launch runs; null when there is none for this type and operator.
+const void* one_gpu_function(int kind, int dtype, int op, int nranks, bool ragged);
+
 // Fused AllReduce (several members in one launch, see batch.cuh). Only the two-shot
 // variants have a fused form; returns null / cudaErrorInvalidDeviceFunction otherwise.
 const void* batch_kernel_function(int variant, int dtype, int op);

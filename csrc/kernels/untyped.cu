@@ -2,6 +2,7 @@
 // AllGather and the single-rank copy, plus their lookup function.
 #define MCCS_UNTYPED_KERNELS 1
 #include "collectives.cuh"
+#include "one_gpu.cuh"
 
 namespace mccs {
 namespace dev {
@@ -15,6 +16,12 @@ extern "C" const void* mccs_kfn_untyped(int variant) {
     case kLocalCopy: return (const void*)&local_copy_kernel;
   }
   return nullptr;
+}
+
+extern "C" const void* mccs_kfn_group_gather(int nranks, int ragged) {
+  if (nranks <= 2) return ragged ? (const void*)&group_gather_ragged_kernel<2> : (const void*)&group_gather_kernel<2>;
+  if (nranks <= 4) return ragged ? (const void*)&group_gather_ragged_kernel<4> : (const void*)&group_gather_kernel<4>;
+  return ragged ? (const void*)&group_gather_ragged_kernel<8> : (const void*)&group_gather_kernel<8>;
 }
 
 }  // namespace dev

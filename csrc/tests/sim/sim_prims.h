@@ -51,6 +51,10 @@ template <int BYTES> inline void st_data(void* p, Raw<BYTES> v) {
   memcpy(p, &v, BYTES);
 }
 
+template <int BYTES> inline Raw<BYTES> ld_local(const void* p) { return ld_data<BYTES>(p); }
+template <int BYTES> inline void st_local(void* p, Raw<BYTES> v) { st_data<BYTES>(p, v); }
+inline uint32_t funnel_right(uint32_t lo, uint32_t hi, uint32_t bits) { return (uint32_t)((((uint64_t)hi << 32) | lo) >> bits); }
+
 // Emulated multicast regions: [base, base + size) stands for the same offsets of every
 // rank's backing buffer.
 // The table may change while kernels of other communicators run (a service binds and

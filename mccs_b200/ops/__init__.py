@@ -40,6 +40,7 @@ VARIANTS = {
     "ag_ring": "AllGather: FIFO-staged ring",
     "rs_direct": "ReduceScatter: every rank loads its block from all peers and reduces it (the reducing half of ar_twoshot)",
     "rs_nvls": "ReduceScatter: multimem.ld_reduce of the own block",
+    "one_gpu": "ranks that share a GPU: every rank's output from every rank's input in one pass over memory, any of the three collectives",
     "local_copy": "single-rank communicator: device copy",
 }
 assert set(VARIANTS) == set(ALGOS)
