@@ -152,7 +152,11 @@ struct CommInitReply {
   uint32_t launch_mode;                   // LaunchMode
   uint32_t fifo_slot_bytes;               // client-side launch: geometry of the ring FIFOs
   uint32_t group_defer;                   // client-side launch: inside a group the library only posts and takes the plans at the end (fused launches are on)
-  uint32_t pad_;
+  // 1: the client lives in the daemon's process and so in its CUDA context: requests name the
+  // caller's stream and the daemon orders against it (or launches on it) itself, without
+  // events in between. `status_va`: the status block whose done_seq tells what has finished.
+  uint32_t caller_streams;
+  uint64_t status_va;
 };
 
 struct CommDestroyReq { Header h; uint64_t comm_handle; };
@@ -230,6 +234,7 @@ union AnyMsg {
 // ---------------------------------------------------------------------------
 enum WrFlags : uint32_t {
   kWrGroupMore = 1u << 0,   // further requests of the same group follow
+  kWrCallerStream = 1u << 1,   // WorkRequest::caller_stream is the stream to order against (CommInitReply::caller_streams)
 };
 
 // Client-side launch: what a rank's proxy hands back for one collective, through the
@@ -285,7 +290,8 @@ struct alignas(64) WorkRequest {
   uint32_t variant;     // Variant requested by the caller (0 = planner decides)
   uint64_t sync_slot;   // mem-op mode: 1 + index of the "submitted" semaphore, 0 = events
   uint64_t sync_value;  // value the caller's stream writes there before this request
-  uint64_t reserved[3];
+  uint64_t caller_stream;   // with kWrCallerStream: the caller's stream itself
+  uint64_t reserved[2];
 };
 static_assert(sizeof(WorkRequest) == kWrBytes, "work request must fill one 128-byte slot");
 
@@ -296,7 +302,8 @@ struct alignas(64) WorkCompletion {
   uint32_t variant;     // what the planner launched
   uint32_t ctas;
   uint64_t comm_seq;    // sequence number of the collective within the communicator
-  uint64_t reserved[4];
+  uint64_t ticket;      // StatusBlock::done_seq once its last kernel has finished (0: nothing was launched)
+  uint64_t reserved[3];
 };
 static_assert(sizeof(WorkCompletion) == kWcBytes, "completion must fill one 64-byte slot");
 

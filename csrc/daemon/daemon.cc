@@ -333,21 +333,39 @@ void Daemon::on_malloc(Session& s, const proto::MallocReq& m) {
   reply(s, r, sizeof(proto::MallocReply), send_fd ? &a.share_fd : nullptr, send_fd ? 1 : 0);
 }
 
+// Kernels on the callers' own streams: the daemon waits for the completion word of the newest
+// one instead of a stream (whose handle is not its own). Every one of them ends, or has reported
+// an error; the bound is for a GPU that has stopped.
+void Daemon::wait_for_caller_streams(Communicator& c) {
+  if (!c.caller_streams || !c.ranks[0] || !c.ranks[0]->status) return;
+  const StatusBlock* st = c.ranks[0]->status;
+  const uint64_t ticket = c.ranks[0]->last_ticket.load(std::memory_order_relaxed);
+  const uint64_t t_end = monotonic_us() + 60ull * 1000 * 1000;
+  while (__atomic_load_n(&st->done_seq, __ATOMIC_ACQUIRE) < ticket && __atomic_load_n(&st->error, __ATOMIC_ACQUIRE) == kDevOk &&
+         monotonic_us() < t_end) {
+    struct timespec ts = {0, 20000};
+    nanosleep(&ts, nullptr);
+  }
+}
+
 void Daemon::quiesce_session_streams(Session& s) {
   // Nothing of this client's communicators may still run on a GPU when memory they
   // use goes away. Kernels are bounded, so this returns.
   std::vector<std::pair<int, void*>> streams;
+  std::vector<Communicator*> comms;   // only this thread destroys communicators
   {
     std::lock_guard<std::mutex> g(mu_);
     for (auto& cr : s.comm_ranks) {
       auto it = comms_.find(cr.first);
       if (it == comms_.end()) continue;
       Communicator& c = *it->second;
+      comms.push_back(&c);
       for (auto& r : c.ranks)
         if (r && r->stream) streams.push_back({r->device, r->stream});
       if (c.group_stream && !c.ranks.empty() && c.ranks[0]) streams.push_back({c.ranks[0]->device, c.group_stream});
     }
   }
+  for (Communicator* c : comms) wait_for_caller_streams(*c);
   for (auto& ds : streams) backend_->stream_sync(ds.first, ds.second);
 }
 
@@ -658,6 +676,8 @@ void Daemon::on_comm_init(Session& s, const proto::CommInitReq& m) {
       r.comm_init_reply.dp_bytes = (uint32_t)rs.dp_bytes;
       r.comm_init_reply.launch_mode = cptr->client_launch ? proto::kLaunchClient : proto::kLaunchDaemon;
       r.comm_init_reply.fifo_slot_bytes = (uint32_t)cptr->fifo_slot_bytes;
+      r.comm_init_reply.caller_streams = cptr->caller_streams ? 1u : 0u;
+      r.comm_init_reply.status_va = cptr->caller_streams ? (uint64_t)cptr->ranks[0]->status : 0;
       r.comm_init_reply.group_defer = cptr->client_launch && cfg_.fuse_allreduce > 1 ? 1u : 0u;
       int fds[2] = {rs.dp_fd, -1};
       int nfds = 1;
@@ -778,6 +798,17 @@ int Daemon::finalize_communicator(Communicator& c) {
     int rc = backend_->stream_create(c.ranks[0]->device, prio, &c.group_stream);
     if (rc != proto::kOk) return rc;
   }
+  // Callers in this process share its CUDA context, so their streams are the daemon's to order
+  // against directly. Not for a tenant with a priority, whose kernels need a stream that has it.
+  bool all_here = true;
+  for (int r = 0; r < c.nranks; r++) all_here &= c.ranks[(size_t)r]->same_process;
+  if (!host && all_here && (c.emulated || c.nranks == 1) && !c.client_launch && prio == 0 && cfg_.sync != "events" &&
+      backend_->memops_supported()) {
+    uint8_t unused[proto::kIpcHandleBytes];
+    int rc = backend_->event_create(c.ranks[0]->device, &c.mark_event, unused);
+    if (rc != proto::kOk) return rc;
+    c.caller_streams = true;
+  }
   std::vector<int> devs(c.devices.begin(), c.devices.end());
   qos_.tenant_register(c.id, devs);
   c.state.store(kCommActive);
@@ -882,6 +913,7 @@ void Daemon::detach_rank(Communicator& c, int rank, int status) {
       if (r && r->status) __atomic_store_n(&r->status->abort, 1u, __ATOMIC_RELEASE);
   if (c.state.load() != kCommInit) proxies_[(size_t)rs->device]->remove_rank(rs);
   rs->gone.store(true);
+  wait_for_caller_streams(c);
   if (rs->stream) backend_->stream_sync(rs->device, rs->stream);
   if (c.group_stream) backend_->stream_sync(rs->device, c.group_stream);
 }
@@ -903,6 +935,8 @@ void Daemon::destroy_communicator(uint32_t comm_id) {
     if (!r->gone.load() && c->state.load() != kCommInit) proxies_[(size_t)r->device]->remove_rank(r.get());
     if (r->stream) { backend_->stream_sync(r->device, r->stream); }
   }
+  wait_for_caller_streams(*c);
+  if (c->mark_event && c->ranks[0]) backend_->event_destroy(c->ranks[0]->device, c->mark_event);
   if (c->group_stream && c->ranks[0]) {
     backend_->stream_sync(c->ranks[0]->device, c->group_stream);
     backend_->stream_destroy(c->ranks[0]->device, c->group_stream);

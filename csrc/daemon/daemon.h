@@ -81,6 +81,8 @@ struct CollOp {
   uint64_t send_va = 0, recv_va = 0;
   uint64_t send_mem = 0, recv_mem = 0, send_off = 0, recv_off = 0;
   void* user_event = nullptr;
+  bool on_caller_stream = false;            // ordered against `caller_stream` by the daemon (see proto::CommInitReply)
+  void* caller_stream = nullptr;
   uint64_t sync_slot = 0, sync_value = 0;   // mem-op mode (see proto::SyncMode)
   uint64_t user_seq = 0;
   uint64_t t_post_us = 0;
@@ -182,6 +184,11 @@ class Communicator {
   std::atomic<bool> paused{false};
   uint64_t created_us = 0;
   void* group_stream = nullptr;   // emulated mode: the one stream that runs all ranks
+  // Clients inside the daemon's process, one GPU: kernels go to the callers' streams. Which
+  // stream the newest kernel went to, and an event for callers on different streams.
+  bool caller_streams = false;
+  void* last_stream = nullptr;
+  void* mark_event = nullptr;
 
   CollSlot slots[kCollSlots];
 
@@ -245,6 +252,10 @@ class ProxyEngine : public Engine {
   bool followers_still_arriving(Communicator& c, CollSlot& s, uint64_t seq);
   bool publish_plan_error(RankState& rs, uint64_t user_seq, int status);
   void order_after_client(RankState& rs, const CollOp& op, void* stream);
+  void order_after_last_launch(Communicator& c, void* stream);
+  void* stream_for_group(Communicator& c, CollSlot& s, uint64_t seq);
+  void begin_group(Communicator& c, CollSlot& s, uint64_t seq, void* stream);
+  void end_group(Communicator& c, CollSlot& s, uint64_t seq, void* stream);
   bool clients_ready(Communicator& c, CollSlot& s, int self_rank);
   void finish_slot(Communicator& c, CollSlot& s, uint64_t seq);
   void housekeeping(RankState& rs);
@@ -335,6 +346,7 @@ class Daemon {
   void detach_rank(Communicator& c, int rank, int status);
   void destroy_communicator(uint32_t comm_id);
   void quiesce_session_streams(Session& s);
+  void wait_for_caller_streams(Communicator& c);
   void proxy_grace_period();
   void drop_mc_regions_using(uint64_t mem_id);
   void admin_loop();

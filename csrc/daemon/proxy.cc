@@ -147,6 +147,8 @@ bool ProxyEngine::post(RankState& rs, const proto::WorkRequest& wr) {
   op.scale = wr.scale;
   op.variant_req = (int)wr.variant;
   op.user_seq = wr.user_seq;
+  op.on_caller_stream = c.caller_streams && (wr.flags & proto::kWrCallerStream) != 0;
+  op.caller_stream = (void*)wr.caller_stream;
   op.sync_slot = wr.sync_slot;
   op.sync_value = wr.sync_value;
   op.send_mem = wr.send_mem; op.send_off = wr.send_off;
@@ -688,12 +690,16 @@ bool ProxyEngine::launch_slices(RankState& rs, CollSlot& s, uint64_t seq) {
       be->event_record(rs.device, rs.backend_event, rs.stream);
     return true;
   }
+  void* const stream = op.on_caller_stream ? op.caller_stream : rs.stream;
   while (rs.next_slice < s.nslices) {
     if (!admit_slice(c, s, rs.next_slice)) return false;
-    if (rs.next_slice == 0) order_after_client(rs, op, rs.stream);
+    if (rs.next_slice == 0) {
+      if (!op.on_caller_stream) order_after_client(rs, op, stream);
+      order_after_last_launch(c, stream);
+    }
     CollArgs a;
     fill_args(c, s, rs.rank, rs.next_slice, &a);
-    int rc = be->launch(rs.device, op.kind, a, s.plan.dims, rs.stream);
+    int rc = be->launch(rs.device, op.kind, a, s.plan.dims, stream);
     if (rc != proto::kOk) {
       c.async_error.store(rc);
       c.state.store(kCommError);
@@ -706,10 +712,12 @@ bool ProxyEngine::launch_slices(RankState& rs, CollSlot& s, uint64_t seq) {
     rs.last_ticket.store(a.seq, std::memory_order_relaxed);
     rs.next_slice++;
   }
-  if (rs.sync.host && op.sync_slot)
-    be->stream_write_value64(rs.device, rs.stream, rs.sync.dev_addr + 8 * proto::kSyncDoneSlot, op.user_seq);
+  if (op.on_caller_stream)
+    ;   // the kernel is on the caller's own stream
+  else if (rs.sync.host && op.sync_slot)
+    be->stream_write_value64(rs.device, stream, rs.sync.dev_addr + 8 * proto::kSyncDoneSlot, op.user_seq);
   else
-    be->event_record(rs.device, rs.backend_event, rs.stream);
+    be->event_record(rs.device, rs.backend_event, stream);
   (void)seq;
   return true;
 }
@@ -759,21 +767,85 @@ void ProxyEngine::signal_done(RankState& rs, uint64_t user_seq, int status) {
   daemon_->backend()->stream_write_value64(rs.device, stream, rs.sync.dev_addr + 8 * proto::kSyncDoneSlot, user_seq);
 }
 
+// Clients inside the daemon's process on one GPU. Collectives of a communicator run in order
+// whatever streams their callers use (its kernels share a counter, and done_seq only grows); on
+// one stream that is given, after a change of stream the new one waits for the last kernel. That
+// wait can only ever sit behind the kernel it waits for, also in a hardware queue that both
+// streams share: the kernel was launched before.
+void ProxyEngine::order_after_last_launch(Communicator& c, void* stream) {
+  if (!c.caller_streams) return;
+  const RankState& r0 = *c.ranks[0];
+  const uint64_t ticket = r0.last_ticket.load(std::memory_order_relaxed);
+  if (c.last_stream != stream && ticket > __atomic_load_n(&r0.status->done_seq, __ATOMIC_ACQUIRE))
+    daemon_->backend()->stream_wait_value64(r0.device, stream, (uint64_t)&r0.status->done_seq, ticket);
+  c.last_stream = stream;
+}
+
+// The stream a launch for all ranks goes to: the caller's, when every rank's caller is on the
+// same one (nothing is queued around the kernel then), else the communicator's own.
+void* ProxyEngine::stream_for_group(Communicator& c, CollSlot& s, uint64_t seq) {
+  const int len = s.fused_kernel ? s.batch_len : 1;
+  for (int k = 0; k < len; k++) {
+    CollSlot& m = k == 0 ? s : c.slot(seq + (uint64_t)k);
+    for (int r = 0; r < c.nranks; r++)
+      if (!m.ops[r].on_caller_stream || m.ops[r].caller_stream != s.ops[0].caller_stream) return c.group_stream;
+  }
+  return s.ops[0].caller_stream;
+}
+
+// Orders `stream` behind what the callers had queued before their requests ...
+void ProxyEngine::begin_group(Communicator& c, CollSlot& s, uint64_t seq, void* stream) {
+  Backend* be = daemon_->backend();
+  const int len = s.fused_kernel ? s.batch_len : 1;
+  for (int k = 0; k < len; k++) {
+    CollSlot& m = k == 0 ? s : c.slot(seq + (uint64_t)k);
+    for (int r = 0; r < c.nranks; r++) {
+      const CollOp& op = m.ops[r];
+      RankState& rr = *c.ranks[(size_t)r];
+      if (!op.on_caller_stream) {
+        order_after_client(rr, op, stream);
+      } else if (op.caller_stream != stream) {
+        be->event_record(rr.device, c.mark_event, op.caller_stream);
+        be->stream_wait_event(rr.device, stream, c.mark_event);
+      }
+    }
+  }
+  order_after_last_launch(c, stream);
+}
+
+// ... and the callers' streams behind the kernel: at once, or through what the client waits for.
+void ProxyEngine::end_group(Communicator& c, CollSlot& s, uint64_t seq, void* stream) {
+  Backend* be = daemon_->backend();
+  bool marked = false;
+  for (int r = 0; r < c.nranks; r++) {
+    const CollOp& op = s.ops[r];
+    RankState& rr = *c.ranks[(size_t)r];
+    if (op.on_caller_stream) {
+      if (op.caller_stream == stream) continue;
+      if (!marked) be->event_record(rr.device, c.mark_event, stream);
+      marked = true;
+      be->stream_wait_event(rr.device, op.caller_stream, c.mark_event);
+    } else if (rr.sync.host && op.sync_slot) {
+      be->stream_write_value64(rr.device, stream, rr.sync.dev_addr + 8 * proto::kSyncDoneSlot,
+                               s.fused_kernel ? last_member_user_seq(c, s, seq, r) : op.user_seq);
+    } else {
+      be->event_record(rr.device, rr.backend_event, stream);
+    }
+  }
+}
+
 // Emulated communicators (all ranks on one GPU) and the host backend run every rank
 // in one launch. Rank 0's proxy issues it; the other ranks wait for it.
 bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
-  (void)seq;
   RankState& r0 = *c.ranks[0];
   Backend* be = daemon_->backend();
+  void* const stream = stream_for_group(c, s, seq);
   if (s.fused_kernel) {
     if (!admit_slice(c, s, 0)) return false;
-    for (int k = 0; k < s.batch_len; k++) {
-      CollSlot& m = k == 0 ? s : c.slot(seq + (uint64_t)k);
-      for (int r = 0; r < c.nranks; r++) order_after_client(*c.ranks[(size_t)r], m.ops[r], c.group_stream);
-    }
+    begin_group(c, s, seq, stream);
     BatchArgs b;
     fill_batch_args(c, s, seq, 0, &b);
-    int rc = be->launch_batch(r0.device, b, s.plan.dims, c.group_stream);
+    int rc = be->launch_batch(r0.device, b, s.plan.dims, stream);
     if (rc != proto::kOk) {
       c.async_error.store(rc);
       c.state.store(kCommError);
@@ -782,25 +854,16 @@ bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
       r0.last_ticket.store(b.base.seq, std::memory_order_relaxed);
     }
     r0.next_slice = 1;
-    for (int r = 0; r < c.nranks; r++) {
-      RankState& rr = *c.ranks[(size_t)r];
-      if (rr.sync.host && s.ops[r].sync_slot)
-        be->stream_write_value64(rr.device, c.group_stream, rr.sync.dev_addr + 8 * proto::kSyncDoneSlot,
-                                 last_member_user_seq(c, s, seq, r));
-      else
-        be->event_record(rr.device, rr.backend_event, c.group_stream);
-    }
+    end_group(c, s, seq, stream);
     s.group_launch.store(2, std::memory_order_release);
     return true;
   }
   while (r0.next_slice < s.nslices) {
     if (!admit_slice(c, s, r0.next_slice)) return false;
-    if (r0.next_slice == 0) {
-      for (int r = 0; r < c.nranks; r++) order_after_client(*c.ranks[(size_t)r], s.ops[r], c.group_stream);
-    }
+    if (r0.next_slice == 0) begin_group(c, s, seq, stream);
     CollArgs a;
     fill_args(c, s, 0, r0.next_slice, &a);
-    int rc = be->launch(r0.device, s.ops[0].kind, a, s.plan.dims, c.group_stream);
+    int rc = be->launch(r0.device, s.ops[0].kind, a, s.plan.dims, stream);
     if (rc != proto::kOk) {
       c.async_error.store(rc);
       c.state.store(kCommError);
@@ -811,13 +874,7 @@ bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
     r0.last_ticket.store(a.seq, std::memory_order_relaxed);
     r0.next_slice++;
   }
-  for (int r = 0; r < c.nranks; r++) {
-    RankState& rr = *c.ranks[(size_t)r];
-    if (rr.sync.host && s.ops[r].sync_slot)
-      be->stream_write_value64(rr.device, c.group_stream, rr.sync.dev_addr + 8 * proto::kSyncDoneSlot, s.ops[r].user_seq);
-    else
-      be->event_record(rr.device, rr.backend_event, c.group_stream);
-  }
+  end_group(c, s, seq, stream);
   s.group_launch.store(2, std::memory_order_release);
   return true;
 }
@@ -956,6 +1013,7 @@ bool ProxyEngine::complete_request(RankState& rs, CollSlot& s, uint64_t seq, int
   wc.variant = (uint32_t)s.plan.variant;
   wc.ctas = (uint32_t)s.plan.dims.ctas;
   wc.comm_seq = seq;
+  if (status == proto::kOk) wc.ticket = s.ticket_base + (uint64_t)s.nslices - 1;
   if (!rs.cq.try_push(&wc)) {
     rs.pending_wc = wc;
     rs.have_pending_wc = true;

@@ -209,7 +209,7 @@ struct Context {
 Context g_ctx;
 
 thread_local int g_group_depth = 0;
-struct GroupItem { struct mccsComm* comm; mccsStream_t stream; };
+struct GroupItem { struct mccsComm* comm; mccsStream_t stream; bool ordered; };   // ordered: the daemon orders the stream itself
 thread_local std::vector<GroupItem> g_group_items;
 
 }  // namespace
@@ -229,6 +229,13 @@ struct mccsComm {
   uint64_t outstanding = 0;      // requests posted whose completion was not read yet
   uint32_t last_variant = 0, last_ctas = 0;
   int sticky_error = 0;
+  // Inside the daemon's process (proto::CommInitReply::caller_streams): the daemon launches on the
+  // caller's stream or orders it itself. `done_seq` and the newest ticket tell whether everything
+  // submitted that way has finished.
+  bool caller_streams = false;
+  const uint64_t* done_seq = nullptr;
+  uint64_t last_ticket = 0;
+  mccsStream_t last_stream = nullptr;   // where the newest of those collectives went
   bool deferred_wait = false;         // collectives do not queue "wait done"; mccsCommWait does
   uint64_t last_posted_seq = 0;       // user_seq of the newest request posted
   pthread_t owner = pthread_self();   // the thread that created (and uses) the communicator
@@ -687,6 +694,7 @@ mccsResult_t wait_completion(mccsComm* comm, proto::WorkCompletion* wc) {
   comm->outstanding--;
   comm->last_variant = wc->variant;
   comm->last_ctas = wc->ctas;
+  if (wc->ticket) comm->last_ticket = wc->ticket;
   if (wc->status != 0 && comm->sticky_error == 0) comm->sticky_error = wc->status;
   return (mccsResult_t)wc->status;
 }
@@ -715,6 +723,7 @@ void reap_completions(mccsComm* comm) {
     comm->outstanding--;
     comm->last_variant = wc.variant;
     comm->last_ctas = wc.ctas;
+    if (wc.ticket) comm->last_ticket = wc.ticket;
     if (wc.status != 0 && comm->sticky_error == 0) comm->sticky_error = wc.status;
   }
 }
@@ -802,7 +811,7 @@ mccsResult_t submit_memops(mccsComm* comm, proto::WorkRequest& wr, mccsStream_t 
     // Inside a group the stream is not made to wait after every collective: the daemon
     // sees all of them submitted at once and queues their kernels back to back;
     // mccsGroupEnd orders the stream after the last one.
-    g_group_items.push_back({comm, stream});
+    g_group_items.push_back({comm, stream, false});
     return mccsSuccess;
   }
   sr = sem_wait_geq(comm, stream, comm->sync_base + 8 * proto::kSyncDoneSlot, wr.user_seq);
@@ -1166,6 +1175,9 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
                     uint64_t recv_bytes, mccsStream_t stream) {
   if (!comm) return mccsInvalidArgument;
   StreamRec* srec = nullptr;
+  // (A deferred wait keeps the collective off the caller's stream; the per-thread default stream
+  // is another one in the daemon's thread.)
+  const bool on_caller_stream = comm->caller_streams && !comm->deferred_wait && stream != (mccsStream_t)CU_STREAM_PER_THREAD;
   {
     std::unique_lock<std::mutex> g(g_ctx.mu);
     if (!g_ctx.connected) return mccsNotConnected;
@@ -1178,7 +1190,7 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
     wr.send_mem = sm->mem_id; wr.send_off = (uint64_t)send - sm->base;
     wr.recv_mem = rm->mem_id; wr.recv_off = (uint64_t)recv - rm->base;
     if (wr.send_off + send_bytes > sm->size || wr.recv_off + recv_bytes > rm->size) return mccsInvalidArgument;
-    if (!comm->sync_base && !comm->client_launch) {
+    if (!comm->sync_base && !comm->client_launch && !on_caller_stream) {
       mccsResult_t r = register_stream_locked(g, comm->device, stream, &srec);
       if (r != mccsSuccess) return r;
     }
@@ -1186,10 +1198,14 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
   if (comm->client_launch) return submit_client_launch(comm, wr, stream);
   if (comm->sync_base) return submit_memops(comm, wr, stream);
   wr.comm_handle = comm->handle;
-  wr.stream_id = srec->stream_id;
+  wr.stream_id = srec ? srec->stream_id : 0;
   wr.user_seq = comm->next_user_seq++;
   if (g_group_depth > 0) wr.flags |= proto::kWrGroupMore;
-  if (g_ctx.backend == proto::kBackendCuda) {
+  if (on_caller_stream) {
+    wr.flags |= proto::kWrCallerStream;
+    wr.caller_stream = (uint64_t)stream;
+    comm->last_stream = stream;
+  } else if (g_ctx.backend == proto::kBackendCuda) {
     CtxScope scope(comm->device);
     if (!scope.ok) return mccsDeviceError;
     CUresult r = g_drv.cuEventRecord_(srec->event, (CUstream)stream);
@@ -1200,12 +1216,13 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
     proto::WorkCompletion wc;
     if (comm->outstanding > 0 && comm->cq.try_pop(&wc)) {
       comm->outstanding--;
+      if (wc.ticket) comm->last_ticket = wc.ticket;
       if (wc.status != 0 && comm->sticky_error == 0) comm->sticky_error = wc.status;
     }
   }
   comm->outstanding++;
   if (g_group_depth > 0) {
-    g_group_items.push_back({comm, stream});
+    g_group_items.push_back({comm, stream, on_caller_stream});
     return mccsSuccess;
   }
   proto::WorkCompletion wc;
@@ -1216,7 +1233,7 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
     if (one != mccsSuccess) r = one;
   }
   if (r != mccsSuccess) return r;
-  if (comm->deferred_wait) return mccsSuccess;
+  if (comm->deferred_wait || on_caller_stream) return mccsSuccess;
   return finish_on_stream(comm, stream);
 }
 
@@ -1455,6 +1472,8 @@ mccsResult_t mccsCommInitRank(mccsComm_t* comm, uint32_t unique_id, int rank, in
   c->client_launch = m.comm_init_reply.launch_mode == proto::kLaunchClient;
   c->group_defer = c->client_launch && m.comm_init_reply.group_defer != 0;
   c->fifo_slot_bytes = m.comm_init_reply.fifo_slot_bytes;
+  c->caller_streams = g_ctx.same_process && m.comm_init_reply.caller_streams != 0 && m.comm_init_reply.status_va != 0 && g_drv.memops;
+  if (c->caller_streams) c->done_seq = &((const StatusBlock*)m.comm_init_reply.status_va)->done_seq;
   if (g_ctx.backend == proto::kBackendHost && m.comm_init_reply.sync_size && fds.size() > 1) {
     const size_t bytes = m.comm_init_reply.sync_size;
     void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_SHARED, fds[1], 0);
@@ -1742,6 +1761,15 @@ mccsResult_t mccsCommWait(mccsComm_t comm, mccsStream_t stream) {
     // "done" only grows and is written in submission order: the newest value covers all.
     return sem_wait_geq(comm, stream, comm->sync_base + 8 * proto::kSyncDoneSlot, comm->last_posted_seq);
   }
+  if (comm->caller_streams && comm->last_ticket && comm->last_stream != stream &&
+      __atomic_load_n(comm->done_seq, __ATOMIC_ACQUIRE) < comm->last_ticket) {
+    // Collectives of a communicator end in order, so the newest ticket covers all of them. The
+    // kernel that raises the word has been launched already (the ticket came with the completion).
+    CtxScope scope(comm->device);
+    if (!scope.ok) return mccsDeviceError;
+    mccsResult_t r = sem_wait_geq(comm, stream, (uint64_t)comm->done_seq, comm->last_ticket);
+    if (r != mccsSuccess) return r;
+  }
   return finish_on_stream(comm, stream);
 }
 
@@ -1765,13 +1793,14 @@ mccsResult_t mccsGroupEnd(void) {
   std::vector<GroupItem> seen;
   for (const GroupItem& it : items) {
     bool dup = false;
-    for (const GroupItem& s : seen) dup |= s.comm == it.comm && s.stream == it.stream;
+    for (const GroupItem& s : seen) dup |= s.comm == it.comm && s.stream == it.stream && s.ordered == it.ordered;
     if (dup) continue;
     seen.push_back(it);
     if (it.comm->sticky_error && result == mccsSuccess) result = (mccsResult_t)it.comm->sticky_error;
     // Event mode: wait for the daemon's "done" event. Mem-op mode: wait for the "done"
     // value of the newest request (values grow in submission order).
-    mccsResult_t r = it.comm->sync_base ? (it.comm->deferred_wait ? mccsSuccess : mccsCommWait(it.comm, it.stream))
+    mccsResult_t r = it.ordered ? mccsSuccess
+                     : it.comm->sync_base ? (it.comm->deferred_wait ? mccsSuccess : mccsCommWait(it.comm, it.stream))
                                         : finish_on_stream(it.comm, it.stream);
     if (r != mccsSuccess) result = r;
   }

@@ -1,0 +1,62 @@
+"""Clients inside the daemon's process whose ranks share a GPU: the daemon launches on the
+caller's stream when all ranks are on one, and orders the callers' streams itself when they are
+not. Long-running work is queued in front of every collective and a consumer behind it, on the
+same stream, on changing streams, on one stream per rank, with a deferred wait and with
+``Communicator.wait`` from another stream: whatever is not ordered reads poisoned values."""
+import threading
+
+import pytest
+import torch
+
+from helpers import fresh_comm_id
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", ["one_stream", "changing", "per_rank", "deferred", "wait_elsewhere"])
+@pytest.mark.parametrize("n", [1, 2, 4])
+def test_collectives_are_ordered_with_the_callers_streams(service, n, mode):
+    M, count = service, 1 << 20
+    torch.cuda.set_device(0)
+    cid, comms = fresh_comm_id(), [None] * n
+    threads = [threading.Thread(target=lambda r=r: comms.__setitem__(r, M.Communicator(cid, r, n, device=0))) for r in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    bufs = [(M.Buffer(count * 4, 0), M.Buffer(count * 4, 0)) for _ in range(n)]
+    send = [a.tensor(torch.float32, count) for a, _ in bufs]
+    recv = [b.tensor(torch.float32, count) for _, b in bufs]
+    streams = [torch.cuda.Stream() for _ in range(max(n, 3))]
+    other = torch.cuda.Stream()
+    big = torch.randn(4096, 4096, device="cuda")
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    for c in comms:
+        c.set_deferred_wait(mode == "deferred")
+    for it in range(12):
+        used = [streams[r if mode == "per_rank" else it % 3 if mode == "changing" else 0] for r in range(n)]
+        for r in range(n):
+            used[r].wait_stream(torch.cuda.default_stream())     # the previous round's consumers
+            with torch.cuda.stream(used[r]):
+                for _ in range(3):
+                    torch.mm(big, big)                           # the inputs exist only after this
+                send[r].fill_(float(it + r))
+                recv[r].fill_(-1.0)
+        with M.group():
+            for r in range(n):
+                comms[r].all_reduce(send[r], recv[r], stream=used[r])
+        for r in range(n):
+            reader = other if mode in ("deferred", "wait_elsewhere") else used[r]
+            if reader is other:
+                comms[r].wait(other)
+            with torch.cuda.stream(reader):
+                wrong = (recv[r] != float(n * it + n * (n - 1) // 2)).sum()
+            torch.cuda.default_stream().wait_stream(reader)
+            bad += wrong
+    torch.cuda.synchronize()
+    assert int(bad) == 0
+    for c in comms:
+        q = c.query()
+        assert q["async_error"] == 0 and q["device_error"] == 0
+        c.destroy()
