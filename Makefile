@@ -29,7 +29,11 @@ HDRS := $(wildcard csrc/*/*.h csrc/*/*.cuh)
 APPS := allreduce_bench allgather_bench allreduce_proto allgather_proto reducescatter_proto traffic_gen ring_config mccs_hello
 APP_BINS := $(addprefix $(OUT)/,$(APPS))
 
-all: $(OUT)/libmccs_daemon.so $(OUT)/libmccs.so $(OUT)/libmccs_kernels.so $(OUT)/mccsd $(OUT)/libmccs_preload.so $(APP_BINS) $(OUT)/host_tests
+# CPython extension of the collective calls, built for the interpreter that runs the package.
+PYTHON  ?= python3
+PYINC   := $(shell $(PYTHON) -c "import sysconfig; print(sysconfig.get_paths()['include'])")
+
+all: $(OUT)/_calls.so $(OUT)/libmccs_daemon.so $(OUT)/libmccs.so $(OUT)/libmccs_kernels.so $(OUT)/mccsd $(OUT)/libmccs_preload.so $(APP_BINS) $(OUT)/host_tests
 
 $(OBJ)/%.o: csrc/%.cc $(HDRS)
 	@mkdir -p $(dir $@)
@@ -73,6 +77,10 @@ $(OUT)/libmccs_kernels.so: $(KLIB_OBJS) csrc/exports_kernels.map
 $(OUT)/libmccs.so: $(SHIM_OBJS) $(EMU_OBJ) csrc/exports.map
 	@mkdir -p $(OUT)
 	$(CXX) -shared -Wl,--version-script=csrc/exports.map -o $@ $(SHIM_OBJS) $(EMU_OBJ) $(LDLIBS)
+
+$(OUT)/_calls.so: csrc/python/calls.cc csrc/include/mccs.h
+	@mkdir -p $(OUT)
+	$(CXX) $(CXXFLAGS) -Wno-missing-field-initializers -I$(PYINC) -shared -o $@ $< -ldl
 
 $(OUT)/libmccs_preload.so: $(OBJ)/shim/preload.o $(OUT)/libmccs.so
 	$(CXX) -shared -Wl,--version-script=csrc/exports_preload.map -o $@ $(OBJ)/shim/preload.o -L$(OUT) -lmccs -Wl,-rpath,'$$ORIGIN' $(LDLIBS)

@@ -1,0 +1,360 @@
+// The calls that issue collectives, as a CPython extension: a Communicator of mccs_b200/client.py
+// holds one CommCalls object and hands its methods out as its own.
+//
+// A collective on a small message costs the GPU a few microseconds; written in Python over ctypes
+// its call alone cost four (keyword handling 0.3, looking up the current stream 1.3, the capture
+// check 0.3, argument objects and the ctypes call 1.5), which n ranks driven by one thread pay n
+// times. Here it is 0.5: the tensor's three properties, one dictionary look-up each for
+// type, operator and variant, and the C call with the interpreter lock released.
+//
+// The C API's functions arrive as addresses (`bind`), so that this module always talks to the
+// libmccs.so the package has loaded and links against nothing.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <cuda.h>
+#include <dlfcn.h>
+#include <stdint.h>
+
+#include "../include/mccs.h"
+
+namespace {
+
+decltype(&mccsAllReduceEx) g_all_reduce;
+decltype(&mccsAllGatherEx) g_all_gather;
+decltype(&mccsReduceScatterEx) g_reduce_scatter;
+decltype(&mccsGroupStart) g_group_start;
+decltype(&mccsGroupEnd) g_group_end;
+
+// Owned for the life of the process.
+PyObject* g_tensor_type;      // torch.Tensor
+PyObject* g_dtypes;           // torch.dtype -> mccsDataType_t
+PyObject* g_ops;              // operator name -> mccsRedOp_t
+PyObject* g_algos;            // variant name -> mccsAlgo_t
+PyObject* g_error;            // MccsError(code, what)
+PyObject* g_buffer_type;      // Buffer
+PyObject* g_current_stream;   // device index -> raw handle of torch's current stream; None without CUDA
+PyObject* g_capturing;        // () -> is the current stream of the current device capturing; None without CUDA
+PyObject *s_data_ptr, *s_numel, *s_element_size, *s_dtype, *s_lower, *s_cuda_stream, *s_ptr;
+
+// The driver calls of the capture check, when libcuda is there.
+decltype(&cuStreamIsCapturing) g_is_capturing;
+decltype(&cuCtxGetDevice) g_ctx_device;
+
+struct Calls {
+  PyObject_HEAD
+  mccsComm_t comm;
+  int device;
+  int cuda;     // the daemon's backend is CUDA
+};
+
+bool is_tensor(PyObject* o) { return PyObject_TypeCheck(o, (PyTypeObject*)g_tensor_type); }
+
+bool to_u64(PyObject* o, uint64_t* out) {   // steals nothing
+  PyObject* i = PyNumber_Index(o);
+  if (!i) {
+    PyErr_Clear();
+    i = PyNumber_Long(o);
+    if (!i) return false;
+  }
+  *out = (uint64_t)PyLong_AsUnsignedLongLongMask(i);
+  Py_DECREF(i);
+  return !PyErr_Occurred();
+}
+
+bool method_u64(PyObject* o, PyObject* name, uint64_t* out) {
+  PyObject* r = PyObject_CallMethodNoArgs(o, name);
+  if (!r) return false;
+  *out = (uint64_t)PyLong_AsUnsignedLongLongMask(r);
+  Py_DECREF(r);
+  return !PyErr_Occurred();
+}
+
+// Address of a tensor, a Buffer or a raw pointer.
+bool address(PyObject* o, uint64_t* out) {
+  if (is_tensor(o)) return method_u64(o, s_data_ptr, out);
+  if (PyObject_TypeCheck(o, (PyTypeObject*)g_buffer_type)) {
+    PyObject* p = PyObject_GetAttr(o, s_ptr);
+    if (!p) return false;
+    const bool ok = to_u64(p, out);
+    Py_DECREF(p);
+    return ok;
+  }
+  return to_u64(o, out);
+}
+
+// dict[key] as an int; KeyError as Python's own subscription raises it.
+bool lookup(PyObject* dict, PyObject* key, int* out) {
+  PyObject* v = PyDict_GetItemWithError(dict, key);
+  if (!v) {
+    if (!PyErr_Occurred()) PyErr_SetObject(PyExc_KeyError, key);
+    return false;
+  }
+  *out = (int)PyLong_AsLong(v);
+  return !(*out == -1 && PyErr_Occurred());
+}
+
+bool op_code(PyObject* op, int* out) {
+  if (PyObject* v = PyDict_GetItemWithError(g_ops, op)) {
+    *out = (int)PyLong_AsLong(v);
+    return true;
+  }
+  if (PyErr_Occurred()) return false;
+  PyObject* low = PyObject_CallMethodNoArgs(op, s_lower);
+  if (!low) return false;
+  const bool ok = lookup(g_ops, low, out);
+  Py_DECREF(low);
+  return ok;
+}
+
+PyObject* raise(int code, const char* what) {
+  PyObject* e = PyObject_CallFunction(g_error, "is", code, what);
+  if (e) {
+    PyErr_SetObject(g_error, e);
+    Py_DECREF(e);
+  }
+  return nullptr;
+}
+
+// The stream a call goes to, and the refusal of graph capture: a collective takes its barrier
+// epoch and its ticket from the daemon at the call, so a graph that captured one would replay
+// stale values.
+bool resolve_stream(Calls* self, PyObject* stream, uint64_t* out) {
+  *out = 0;
+  if (self->cuda) {
+    PyObject* dev = PyLong_FromLong(self->device);
+    PyObject* cur = dev ? PyObject_CallOneArg(g_current_stream, dev) : nullptr;
+    Py_XDECREF(dev);
+    if (!cur) return false;
+    const uint64_t current = (uint64_t)PyLong_AsUnsignedLongLongMask(cur);
+    Py_DECREF(cur);
+    bool capturing = false, known = false;
+    CUdevice now = -1;
+    if (g_is_capturing && g_ctx_device && g_ctx_device(&now) == CUDA_SUCCESS && (int)now == self->device) {
+      CUstreamCaptureStatus st = CU_STREAM_CAPTURE_STATUS_NONE;
+      known = g_is_capturing((CUstream)current, &st) == CUDA_SUCCESS;
+      capturing = known && st != CU_STREAM_CAPTURE_STATUS_NONE;
+    }
+    if (!known) {   // another device is current, or the question was refused: as torch answers it
+      PyObject* c = PyObject_CallNoArgs(g_capturing);
+      if (!c) PyErr_Clear();   // no usable CUDA runtime in this process: nothing can be capturing
+      else { capturing = PyObject_IsTrue(c) == 1; Py_DECREF(c); }
+    }
+    if (capturing) { raise(mccsUnsupported, "a collective inside CUDA graph capture"); return false; }
+    *out = current;
+  }
+  if (stream && stream != Py_None) {
+    if (PyLong_Check(stream)) { *out = (uint64_t)PyLong_AsUnsignedLongLongMask(stream); return !PyErr_Occurred(); }
+    PyObject* h = PyObject_GetAttr(stream, s_cuda_stream);
+    if (!h) return false;
+    const bool ok = to_u64(h, out);
+    Py_DECREF(h);
+    return ok;
+  }
+  return true;
+}
+
+// Arguments of a METH_FASTCALL | METH_KEYWORDS method by name; `npos` of them may be positional.
+bool take(const char* fn, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames, const char* const* names, int npos, int nrequired,
+          int total, PyObject** out) {
+  if (nargs > npos) {
+    PyErr_Format(PyExc_TypeError, "%s() takes at most %d positional arguments (%zd given)", fn, npos, nargs);
+    return false;
+  }
+  for (Py_ssize_t i = 0; i < nargs; i++) out[i] = args[i];
+  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  for (Py_ssize_t k = 0; k < nkw; k++) {
+    PyObject* name = PyTuple_GET_ITEM(kwnames, k);
+    int at = -1;
+    for (int i = 0; i < total && at < 0; i++)
+      if (PyUnicode_CompareWithASCIIString(name, names[i]) == 0) at = i;
+    if (at < 0) { PyErr_Format(PyExc_TypeError, "%s() got an unexpected keyword argument '%U'", fn, name); return false; }
+    if (out[at]) { PyErr_Format(PyExc_TypeError, "%s() got multiple values for argument '%U'", fn, name); return false; }
+    out[at] = args[nargs + k];
+  }
+  for (int i = 0; i < nrequired; i++)
+    if (!out[i]) { PyErr_Format(PyExc_TypeError, "%s() missing required argument '%s'", fn, names[i]); return false; }
+  return true;
+}
+
+bool given(PyObject* o) { return o && o != Py_None; }
+
+// all_reduce and reduce_scatter: `from_send`: whether send (else recv) names type and count.
+PyObject* reducing(Calls* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames, const char* fn, const char* what, bool scatter) {
+  static const char* const names[] = {"send", "recv", "count", "dtype", "op", "scale", "algo", "stream"};
+  PyObject* a[8] = {nullptr};
+  if (!take(fn, args, nargs, kwnames, names, 2, scatter ? 2 : 1, 8, a)) return nullptr;
+  PyObject* recv = given(a[1]) || scatter ? a[1] : a[0];
+  PyObject* shape = scatter ? recv : a[0];
+  uint64_t send_va, recv_va, count = 0;
+  int dtype = 0, op = mccsSum, algo = mccsAlgoAuto;
+  bool have_count = given(a[2]), have_dtype = given(a[3]);
+  if (have_count && !to_u64(a[2], &count)) return nullptr;
+  if (have_dtype && !lookup(g_dtypes, a[3], &dtype)) return nullptr;
+  if (is_tensor(shape)) {
+    if (!have_count && !method_u64(shape, s_numel, &count)) return nullptr;
+    if (!have_dtype) {
+      PyObject* d = PyObject_GetAttr(shape, s_dtype);
+      if (!d) return nullptr;
+      const bool ok = lookup(g_dtypes, d, &dtype);
+      Py_DECREF(d);
+      if (!ok) return nullptr;
+    }
+  } else if (!have_count || !have_dtype) {
+    PyErr_SetString(PyExc_ValueError, "dtype and count are needed for raw pointers");
+    return nullptr;
+  }
+  float scale = 1.0f;
+  if (a[5]) {
+    const double d = PyFloat_AsDouble(a[5]);
+    if (d == -1.0 && PyErr_Occurred()) return nullptr;
+    scale = (float)d;
+  }
+  if (a[4] && !op_code(a[4], &op)) return nullptr;
+  if (a[6] && !lookup(g_algos, a[6], &algo)) return nullptr;
+  if (!address(a[0], &send_va)) return nullptr;
+  if (recv == a[0]) recv_va = send_va;
+  else if (!address(recv, &recv_va)) return nullptr;
+  uint64_t stream;
+  if (!resolve_stream(self, a[7], &stream)) return nullptr;
+  mccsResult_t rc;
+  const mccsComm_t comm = self->comm;
+  Py_BEGIN_ALLOW_THREADS
+  rc = (scatter ? g_reduce_scatter : g_all_reduce)(comm, (const void*)send_va, (void*)recv_va, (size_t)count, (mccsDataType_t)dtype, (mccsRedOp_t)op,
+                                                   scale, (mccsAlgo_t)algo, (mccsStream_t)stream);
+  Py_END_ALLOW_THREADS
+  if (rc != mccsSuccess) return raise(rc, what);
+  Py_RETURN_NONE;
+}
+
+PyObject* calls_all_reduce(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  return reducing((Calls*)self, args, nargs, kwnames, "all_reduce", "mccsAllReduce", false);
+}
+
+PyObject* calls_reduce_scatter(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  return reducing((Calls*)self, args, nargs, kwnames, "reduce_scatter", "mccsReduceScatter", true);
+}
+
+PyObject* calls_all_gather(PyObject* self_, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  static const char* const names[] = {"send", "recv", "nbytes", "algo", "stream"};
+  Calls* self = (Calls*)self_;
+  PyObject* a[5] = {nullptr};
+  if (!take("all_gather", args, nargs, kwnames, names, 2, 2, 5, a)) return nullptr;
+  uint64_t nbytes = 0, send_va, recv_va, stream;
+  if (given(a[2])) {
+    if (!to_u64(a[2], &nbytes)) return nullptr;
+  } else if (is_tensor(a[0])) {
+    uint64_t n = 0, esz = 0;
+    if (!method_u64(a[0], s_numel, &n) || !method_u64(a[0], s_element_size, &esz)) return nullptr;
+    nbytes = n * esz;
+  } else {
+    PyErr_SetString(PyExc_ValueError, "nbytes is needed for raw pointers");
+    return nullptr;
+  }
+  int algo = mccsAlgoAuto;
+  if (a[3] && !lookup(g_algos, a[3], &algo)) return nullptr;
+  if (!address(a[0], &send_va) || !address(a[1], &recv_va)) return nullptr;
+  if (!resolve_stream(self, a[4], &stream)) return nullptr;
+  mccsResult_t rc;
+  const mccsComm_t comm = self->comm;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_all_gather(comm, (const void*)send_va, (void*)recv_va, (size_t)nbytes, (mccsAlgo_t)algo, (mccsStream_t)stream);
+  Py_END_ALLOW_THREADS
+  if (rc != mccsSuccess) return raise(rc, "mccsAllGather");
+  Py_RETURN_NONE;
+}
+
+PyObject* calls_attach(PyObject* self_, PyObject* args) {
+  Calls* self = (Calls*)self_;
+  unsigned long long h = 0;
+  if (!PyArg_ParseTuple(args, "Kii", &h, &self->device, &self->cuda)) return nullptr;
+  self->comm = (mccsComm_t)h;
+  Py_RETURN_NONE;
+}
+
+PyMethodDef calls_methods[] = {
+    {"all_reduce", (PyCFunction)(void (*)(void))calls_all_reduce, METH_FASTCALL | METH_KEYWORDS,
+     "all_reduce(send, recv=None, *, count=None, dtype=None, op='sum', scale=1.0, algo='auto', stream=None)\n"
+     "AllReduce ``count`` elements; in place when ``recv`` is None."},
+    {"all_gather", (PyCFunction)(void (*)(void))calls_all_gather, METH_FASTCALL | METH_KEYWORDS,
+     "all_gather(send, recv, *, nbytes=None, algo='auto', stream=None)\n"
+     "AllGather ``nbytes`` per rank into ``recv`` (``nranks * nbytes`` bytes)."},
+    {"reduce_scatter", (PyCFunction)(void (*)(void))calls_reduce_scatter, METH_FASTCALL | METH_KEYWORDS,
+     "reduce_scatter(send, recv, *, count=None, dtype=None, op='sum', scale=1.0, algo='auto', stream=None)\n"
+     "ReduceScatter: ``send`` holds ``nranks * count`` elements, ``recv`` receives the reduction of block ``rank``\n"
+     "(``count`` elements). In place when ``recv`` is the rank's own block of ``send``. The reference has no such call."},
+    {"_attach", calls_attach, METH_VARARGS, "_attach(handle, device, is_cuda): the communicator the calls go to (handle 0: none)"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyTypeObject calls_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyObject* module_group_start(PyObject*, PyObject*) {
+  const mccsResult_t rc = g_group_start();
+  if (rc != mccsSuccess) return raise(rc, "mccsGroupStart");
+  Py_RETURN_NONE;
+}
+
+// group_end(quiet): `quiet` when an exception is on its way out of the block already.
+PyObject* module_group_end(PyObject*, PyObject* quiet) {
+  mccsResult_t rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_group_end();
+  Py_END_ALLOW_THREADS
+  if (rc != mccsSuccess && quiet != Py_True) return raise(rc, "mccsGroupEnd");
+  Py_RETURN_NONE;
+}
+
+// bind(functions, tensor type, Buffer, dtypes, ops, algos, MccsError, current stream, capturing)
+PyObject* module_bind(PyObject*, PyObject* args) {
+  unsigned long long ar, ag, rs, gs, ge;
+  PyObject *tensor, *buffer, *dtypes, *ops, *algos, *error, *current, *capturing;
+  if (!PyArg_ParseTuple(args, "(KKKKK)OOO!O!O!OOO", &ar, &ag, &rs, &gs, &ge, &tensor, &buffer, &PyDict_Type, &dtypes, &PyDict_Type, &ops,
+                        &PyDict_Type, &algos, &error, &current, &capturing))
+    return nullptr;
+  g_all_reduce = (decltype(g_all_reduce))ar;
+  g_all_gather = (decltype(g_all_gather))ag;
+  g_reduce_scatter = (decltype(g_reduce_scatter))rs;
+  g_group_start = (decltype(g_group_start))gs;
+  g_group_end = (decltype(g_group_end))ge;
+  g_tensor_type = Py_NewRef(tensor);
+  g_buffer_type = Py_NewRef(buffer);
+  g_dtypes = Py_NewRef(dtypes);
+  g_ops = Py_NewRef(ops);
+  g_algos = Py_NewRef(algos);
+  g_error = Py_NewRef(error);
+  g_current_stream = Py_NewRef(current);
+  g_capturing = Py_NewRef(capturing);
+  if (void* lib = dlopen("libcuda.so.1", RTLD_NOW | RTLD_LOCAL)) {
+    g_is_capturing = (decltype(g_is_capturing))dlsym(lib, "cuStreamIsCapturing");
+    g_ctx_device = (decltype(g_ctx_device))dlsym(lib, "cuCtxGetDevice");
+  }
+  Py_RETURN_NONE;
+}
+
+PyMethodDef module_methods[] = {{"bind", module_bind, METH_VARARGS, nullptr},
+                                {"group_start", module_group_start, METH_NOARGS, nullptr},
+                                {"group_end", module_group_end, METH_O, nullptr},
+                                {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_calls", "Collective calls of mccs_b200.", -1, module_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__calls(void) {
+  calls_type.tp_name = "mccs_b200._calls.CommCalls";
+  calls_type.tp_basicsize = sizeof(Calls);
+  calls_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  calls_type.tp_methods = calls_methods;
+  calls_type.tp_new = PyType_GenericNew;
+  if (PyType_Ready(&calls_type) < 0) return nullptr;
+  s_data_ptr = PyUnicode_InternFromString("data_ptr");
+  s_numel = PyUnicode_InternFromString("numel");
+  s_element_size = PyUnicode_InternFromString("element_size");
+  s_dtype = PyUnicode_InternFromString("dtype");
+  s_lower = PyUnicode_InternFromString("lower");
+  s_cuda_stream = PyUnicode_InternFromString("cuda_stream");
+  s_ptr = PyUnicode_InternFromString("ptr");
+  PyObject* m = PyModule_Create(&module_def);
+  if (!m) return nullptr;
+  PyModule_AddObject(m, "CommCalls", Py_NewRef((PyObject*)&calls_type));
+  return m;
+}

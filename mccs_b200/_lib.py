@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from ctypes import (POINTER, Structure, byref, c_char_p, c_float, c_int, c_int32, c_size_t,
                     c_uint32, c_uint64, c_void_p)
 
@@ -116,6 +117,40 @@ def daemon_lib() -> ctypes.CDLL:
     return lib
 
 
+_calls = None
+_calls_lock = threading.Lock()
+
+
+def calls():
+    """The CPython extension of the collective calls (``csrc/python/calls.cc``), bound to the
+    shim's functions."""
+    global _calls
+    if _calls is not None:
+        return _calls
+    with _calls_lock:
+        if _calls is not None:
+            return _calls
+        import importlib.machinery
+        import importlib.util
+
+        import torch
+
+        from . import client
+        path = os.path.join(NATIVE_DIR, "_calls.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build the native code with `make -j` at the repository root")
+        loader = importlib.machinery.ExtensionFileLoader("mccs_b200._calls", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("mccs_b200._calls", loader))
+        loader.exec_module(mod)
+        lib = shim()
+        mod.bind(tuple(ctypes.cast(getattr(lib, f), c_void_p).value for f in
+                       ("mccsAllReduceEx", "mccsAllGatherEx", "mccsReduceScatterEx", "mccsGroupStart", "mccsGroupEnd")),
+                 torch.Tensor, client.Buffer, client.DTYPES, client.OPS, client.ALGOS, MccsError,
+                 getattr(torch._C, "_cuda_getCurrentRawStream", None), torch.cuda.is_current_stream_capturing)
+        _calls = mod
+    return _calls
+
+
 class MccsError(RuntimeError):
     def __init__(self, code: int, what: str):
         self.code = code
@@ -128,4 +163,4 @@ def check(code: int, what: str) -> None:
         raise MccsError(code, what)
 
 
-__all__ = ["shim", "daemon_lib", "check", "MccsError", "CommInfo", "NATIVE_DIR", "byref"]
+__all__ = ["shim", "daemon_lib", "calls", "check", "MccsError", "CommInfo", "NATIVE_DIR", "byref"]

@@ -11,7 +11,7 @@ from __future__ import annotations
 import ctypes
 import json
 from ctypes import byref, c_uint32, c_uint64, c_void_p
-from typing import Optional, Sequence, Union
+from typing import Optional, Sequence
 
 import torch
 
@@ -114,14 +114,6 @@ class Buffer:
             pass
 
 
-def _ptr(x: Union[torch.Tensor, Buffer, int]) -> int:
-    if isinstance(x, torch.Tensor):
-        return x.data_ptr()
-    if isinstance(x, Buffer):
-        return x.ptr
-    return int(x)
-
-
 def _stream_handle(stream) -> Optional[int]:
     if stream is None:
         return None
@@ -147,11 +139,17 @@ class Communicator:
 
     def __init__(self, unique_id: int, rank: int, nranks: int, device: int = 0, root_addr: str = "127.0.0.1"):
         h = c_void_p()
+        self._calls = _lib.calls().CommCalls()
         check(_lib.shim().mccsCommInitRank(byref(h), int(unique_id), int(rank), int(nranks), int(device),
                                            root_addr.encode()), "mccsCommInitRank")
         self._h = h
         self.unique_id, self.rank, self.nranks, self.device = int(unique_id), int(rank), int(nranks), int(device)
         self._is_cuda = backend() == "cuda"
+        self._calls._attach(h.value, self.device, 1 if self._is_cuda else 0)
+        # unless a subclass has its own
+        for name in ("all_reduce", "all_gather", "reduce_scatter"):
+            if getattr(type(self), name) is getattr(Communicator, name):
+                setattr(self, name, getattr(self._calls, name))
 
     @property
     def handle(self) -> int:
@@ -166,42 +164,23 @@ class Communicator:
             return int(torch.cuda.current_stream(self.device).cuda_stream)
         return None
 
+    # The three collectives. Every instance carries the native calls under the same names (see
+    # __init__), so these bodies only run for a subclass that reaches them through super().
     def all_reduce(self, send, recv=None, *, count: Optional[int] = None, dtype: Optional[torch.dtype] = None,
                    op: str = "sum", scale: float = 1.0, algo: str = "auto", stream=None) -> None:
         """AllReduce ``count`` elements; in place when ``recv`` is None."""
-        if recv is None:
-            recv = send
-        if isinstance(send, torch.Tensor):
-            dtype = dtype or send.dtype
-            count = send.numel() if count is None else count
-        if dtype is None or count is None:
-            raise ValueError("dtype and count are needed for raw pointers")
-        check(_lib.shim().mccsAllReduceEx(self._h, c_void_p(_ptr(send)), c_void_p(_ptr(recv)), int(count),
-                                          DTYPES[dtype], OPS[op.lower()], float(scale), ALGOS[algo],
-                                          c_void_p(self._stream(stream))), "mccsAllReduce")
+        self._calls.all_reduce(send, recv, count=count, dtype=dtype, op=op, scale=scale, algo=algo, stream=stream)
 
     def all_gather(self, send, recv, *, nbytes: Optional[int] = None, algo: str = "auto", stream=None) -> None:
         """AllGather ``nbytes`` per rank into ``recv`` (``nranks * nbytes`` bytes)."""
-        if nbytes is None:
-            if not isinstance(send, torch.Tensor):
-                raise ValueError("nbytes is needed for raw pointers")
-            nbytes = send.numel() * send.element_size()
-        check(_lib.shim().mccsAllGatherEx(self._h, c_void_p(_ptr(send)), c_void_p(_ptr(recv)), int(nbytes),
-                                          ALGOS[algo], c_void_p(self._stream(stream))), "mccsAllGather")
+        self._calls.all_gather(send, recv, nbytes=nbytes, algo=algo, stream=stream)
 
     def reduce_scatter(self, send, recv, *, count: Optional[int] = None, dtype: Optional[torch.dtype] = None,
                        op: str = "sum", scale: float = 1.0, algo: str = "auto", stream=None) -> None:
         """ReduceScatter: ``send`` holds ``nranks * count`` elements, ``recv`` receives the
         reduction of block ``rank`` (``count`` elements). In place when ``recv`` is the
         rank's own block of ``send``. The reference has no such call."""
-        if isinstance(recv, torch.Tensor):
-            dtype = dtype or recv.dtype
-            count = recv.numel() if count is None else count
-        if dtype is None or count is None:
-            raise ValueError("dtype and count are needed for raw pointers")
-        check(_lib.shim().mccsReduceScatterEx(self._h, c_void_p(_ptr(send)), c_void_p(_ptr(recv)), int(count),
-                                              DTYPES[dtype], OPS[op.lower()], float(scale), ALGOS[algo],
-                                              c_void_p(self._stream(stream))), "mccsReduceScatter")
+        self._calls.reduce_scatter(send, recv, count=count, dtype=dtype, op=op, scale=scale, algo=algo, stream=stream)
 
     def set_deferred_wait(self, on: bool) -> None:
         """With deferred waiting a collective call does not make the caller's stream wait
@@ -238,6 +217,7 @@ class Communicator:
 
     def destroy(self) -> None:
         if self._h is not None and self._h.value:
+            self._calls._attach(0, self.device, 0)
             _lib.shim().mccsCommDestroy(self._h)
             self._h = c_void_p()
 
@@ -252,13 +232,11 @@ class group:
     """``with group():`` submits the enclosed collectives back to back (GroupCall)."""
 
     def __enter__(self):
-        check(_lib.shim().mccsGroupStart(), "mccsGroupStart")
+        _lib.calls().group_start()
         return self
 
     def __exit__(self, *exc):
-        rc = _lib.shim().mccsGroupEnd()
-        if exc[0] is None:
-            check(rc, "mccsGroupEnd")
+        _lib.calls().group_end(exc[0] is not None)
 
 
 def admin_request(port: int, body: dict, *, host: str = "127.0.0.1", type_: int = 2) -> dict:
