@@ -331,7 +331,9 @@ bool ProxyEngine::plan_slot(Communicator& c, CollSlot& s, uint64_t seq) {
     }
   }
   const uint64_t now = monotonic_us();
-  in.cta_cap = daemon_->qos().cta_cap(c.id, now);
+  bool one_stream = o0.on_caller_stream;   // the kernel goes to this stream of the caller's (see stream_for_group)
+  for (int r = 1; r < c.nranks; r++) one_stream &= s.ops[r].on_caller_stream && s.ops[r].caller_stream == o0.caller_stream;
+  in.cta_cap = daemon_->qos().cta_cap(c.id, now, one_stream ? (uint64_t)o0.caller_stream + 1 : 0);
 
   Plan plan = daemon_->planner().plan(in);
   for (int attempt = 0; attempt < 3 && plan.status == proto::kOk; attempt++) {

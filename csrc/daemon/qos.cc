@@ -79,15 +79,17 @@ int QosArbiter::contenders(uint32_t id, uint64_t now_us) {
   return n;
 }
 
-int QosArbiter::cta_cap(uint32_t id, uint64_t now_us) {
+int QosArbiter::cta_cap(uint32_t id, uint64_t now_us, uint64_t stream) {
   std::lock_guard<std::mutex> g(mu_);
-  if (!enabled_) return 0;
   Tenant& me = tenant(id);
+  me.stream = stream;
+  if (!enabled_) return 0;
   if (me.cfg.cta_quota > 0) return me.cfg.cta_quota;
   double total = me.cfg.weight;
   int others = 0;
   for (const auto& kv : tenants_) {
     if (kv.first == id || !is_contender(kv.second, now_us) || !shares_device(me, kv.second)) continue;
+    if (stream != 0 && kv.second.stream == stream) continue;
     total += kv.second.cfg.weight;
     others++;
   }

@@ -53,8 +53,10 @@ class QosArbiter {
 
   // Tenants other than `id` that share a device with it and were active recently.
   int contenders(uint32_t id, uint64_t now_us);
-  // CTA cap for a collective planned now (0 = no cap).
-  int cta_cap(uint32_t id, uint64_t now_us);
+  // CTA cap for a collective planned now (0 = no cap). `stream`: which stream its kernel will
+  // go to (0: one of the communicator's own). Contenders whose kernels go to the same stream
+  // never run beside this one, so they take no share of the SMs from it.
+  int cta_cap(uint32_t id, uint64_t now_us, uint64_t stream = 0);
   // Bytes per time slice for a collective planned now (0 = do not slice).
   uint64_t slice_bytes(uint32_t id, uint64_t now_us);
   int stream_priority(uint32_t id);   // 0 normal, 1 high
@@ -84,6 +86,7 @@ class QosArbiter {
     uint64_t outstanding_bytes = 0;
     int inflight_ctas = 0;           // most CTAs any launch in flight uses per GPU (a tenant's launches run one after another)
     uint64_t deferred_residency = 0;
+    uint64_t stream = 0;             // where its newest collective goes (see cta_cap)
     uint64_t last_active_us = 0;
     uint64_t waiting_since_us = 0;   // 0: nothing waiting
     uint64_t round = 0;
