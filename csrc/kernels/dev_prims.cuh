@@ -181,6 +181,9 @@ template <> __device__ __forceinline__ void st_local<8>(void* p, Raw<8> v) {
 template <> __device__ __forceinline__ void st_local<16>(void* p, Raw<16> v) {
   asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
 }
+// Waits for the kernel in front of this one on the stream, when this one was launched while that
+// was still draining (launch_local in launch.cu); nothing otherwise.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The low word of (hi:lo) >> bits, 0 <= bits < 32.
 __device__ __forceinline__ uint32_t funnel_right(uint32_t lo, uint32_t hi, uint32_t bits) { return __funnelshift_r(lo, hi, bits); }
 

@@ -137,6 +137,23 @@ int max_cooperative_ctas(int variant, int dtype, int op, int threads, int nranks
   return sms * per_sm / nranks;
 }
 
+// Launch of a kernel that no other GPU takes part in. It may be set up while the kernel in front of
+// it on the stream is still draining (it waits for that one's end in its first instruction): 1 to 2 us
+// less between two kernels of a stream.
+static cudaError_t launch_local(const void* fn, dim3 grid, dim3 block, void** params, void* stream) {
+  cudaLaunchAttribute overlap;
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = (cudaStream_t)stream;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, fn, params);
+}
+
 cudaError_t launch_one_gpu(int kind, const CollArgs& args, int max_ctas, bool completion, void* stream) {
   const int n = args.nranks;
   if (n < 2 || n > kMaxRanks) return cudaErrorInvalidValue;
@@ -185,7 +202,7 @@ cudaError_t launch_one_gpu(int kind, const CollArgs& args, int max_ctas, bool co
   if (ctas < 1) ctas = 1;
   if (ctas > 0x7fffffffull) ctas = 0x7fffffffull;
   void* params[] = {(void*)&a};
-  return cudaLaunchKernel(fn, dim3((unsigned)ctas, (unsigned)groups, 1u), dim3((unsigned)threads, 1u, 1u), params, 0, (cudaStream_t)stream);
+  return launch_local(fn, dim3((unsigned)ctas, (unsigned)groups, 1u), dim3((unsigned)threads, 1u, 1u), params, stream);
 }
 
 cudaError_t launch_collective(int kind, const CollArgs& args, LaunchDims dims, void* stream) {
@@ -208,6 +225,7 @@ cudaError_t launch_collective(int kind, const CollArgs& args, LaunchDims dims, v
   dim3 grid((unsigned)dims.ctas, a.emulated ? (unsigned)a.nranks : 1u, 1u);
   dim3 block((unsigned)dims.threads, 1u, 1u);
   void* params[] = {(void*)&a};
+  if (a.variant == kLocalCopy) return launch_local(fn, grid, block, params, stream);
   if (a.emulated && a.nranks > 1) {
     // All ranks' CTAs wait on one another, so they must be resident together.
     return cudaLaunchCooperativeKernel(fn, grid, block, params, 0, (cudaStream_t)stream);

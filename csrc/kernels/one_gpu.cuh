@@ -85,6 +85,7 @@ __device__ __forceinline__ void one_gpu_finish(const OneGpuArgs& a) {
 }
 
 __device__ __forceinline__ void one_gpu_begin(const OneGpuArgs& a) {
+  wait_for_previous_kernel();
   if (a.trace && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     const uint64_t t = globaltimer_ns();
     for (int r = 0; r < a.nranks; r++) st_relaxed_sys_u64(&a.status[r]->start_ns, t);

@@ -53,6 +53,7 @@ template <int BYTES> inline void st_data(void* p, Raw<BYTES> v) {
 
 template <int BYTES> inline Raw<BYTES> ld_local(const void* p) { return ld_data<BYTES>(p); }
 template <int BYTES> inline void st_local(void* p, Raw<BYTES> v) { st_data<BYTES>(p, v); }
+inline void wait_for_previous_kernel() {}
 inline uint32_t funnel_right(uint32_t lo, uint32_t hi, uint32_t bits) { return (uint32_t)((((uint64_t)hi << 32) | lo) >> bits); }
 
 // Emulated multicast regions: [base, base + size) stands for the same offsets of every
