@@ -234,6 +234,10 @@ union AnyMsg {
 // ---------------------------------------------------------------------------
 enum WrFlags : uint32_t {
   kWrGroupMore = 1u << 0,   // further requests of the same group follow
+  // The buffers are no allocations of the service: send_off / recv_off are the caller's own
+  // addresses. Only for a communicator of one rank whose kernels the caller's process launches
+  // (itself, or through a daemon inside it): nobody else ever addresses them.
+  kWrExternal = 1u << 2,
   kWrCallerStream = 1u << 1,   // WorkRequest::caller_stream is the stream to order against (CommInitReply::caller_streams)
 };
 

@@ -166,7 +166,16 @@ bool ProxyEngine::post(RankState& rs, const proto::WorkRequest& wr) {
     const uint64_t send_bytes = send_units(op.kind, op.count, c.nranks) * esz;
     const uint64_t recv_bytes = recv_units(op.kind, op.count, c.nranks) * esz;
     int sdev = -1, rdev = -1;
-    if (!daemon_->translate(rs.session_id, op.send_mem, op.send_off, send_bytes, &op.send_va, &sdev)) {
+    if (wr.flags & proto::kWrExternal) {
+      if (c.nranks == 1 && (c.client_launch || op.on_caller_stream)) {
+        op.send_mem = op.recv_mem = 0;
+        op.send_va = wr.send_off;
+        op.recv_va = wr.recv_off;
+        sdev = rdev = rs.device;
+      } else {
+        status = proto::kErrInvalidArgument;
+      }
+    } else if (!daemon_->translate(rs.session_id, op.send_mem, op.send_off, send_bytes, &op.send_va, &sdev)) {
       status = proto::kErrNotFound;
     } else if (!daemon_->translate(rs.session_id, op.recv_mem, op.recv_off, recv_bytes, &op.recv_va, &rdev)) {
       daemon_->release_mem_ref(op.send_mem);

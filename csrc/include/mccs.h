@@ -146,6 +146,14 @@ mccsResult_t mccsReduceScatterEx(mccsComm_t comm, const void* send, void* recv, 
                                  mccsDataType_t dtype, mccsRedOp_t op, float scale, mccsAlgo_t algo,
                                  mccsStream_t stream);
 
+/* A communicator of one rank: every collective is a copy of `bytes` bytes from `send` to `recv`
+ * (nothing when they are equal). Unlike the collective calls this takes any memory of the
+ * communicator's GPU, because no other process ever addresses it; it is planned, admitted and counted
+ * like them. mccsCommTakesAnyMemory tells whether a communicator can (1) or not (0: more ranks, no
+ * GPU, or a daemon in another process that launches the kernels), mccsUnsupported otherwise. */
+int mccsCommTakesAnyMemory(mccsComm_t comm);
+mccsResult_t mccsCommSelfCopy(mccsComm_t comm, const void* send, void* recv, size_t bytes, mccsStream_t stream);
+
 /* Deferred waiting. By default every collective call also makes the caller's stream wait
  * for the collective (stream order, like a kernel launch). A caller that issues many
  * collectives from a side stream and only needs the results later (gradient buckets

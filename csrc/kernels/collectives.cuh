@@ -549,6 +549,45 @@ __global__ void __launch_bounds__(kMaxThreads) ag_direct_kernel(const __grid_con
   finish(a, rank);
 }
 
+// ----------------------------------------------------------------------------
+// Buffers at any alignment, for the kernels that stay on one GPU.
+// ----------------------------------------------------------------------------
+// The 16 bytes at `p`, which lies `shift` bytes (0..15) behind a 16-byte boundary. `shift` is
+// the same in the whole grid. Both aligned packs that are read hold at least one byte of the
+// 16, so neither lies outside the page of the data.
+__device__ __forceinline__ Raw<16> ld_shifted(const char* p, uint32_t shift) {
+  const char* q = p - shift;
+  const Raw<16> lo = ld_local<16>(q);
+  if (shift == 0) return lo;
+  const Raw<16> hi = ld_local<16>(q + 16);
+  uint32_t w0 = lo.x, w1 = lo.y, w2 = lo.z, w3 = lo.w, w4 = hi.x;
+  if (shift & 8u) { w0 = lo.z; w1 = lo.w; w2 = hi.x; w3 = hi.y; w4 = hi.z; }
+  uint32_t w5 = (shift & 8u) ? hi.w : hi.y;
+  if (shift & 4u) { w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; }
+  const uint32_t bits = (shift & 3u) * 8u;
+  Raw<16> r;
+  r.x = funnel_right(w0, w1, bits);
+  r.y = funnel_right(w1, w2, bits);
+  r.z = funnel_right(w2, w3, bits);
+  r.w = funnel_right(w3, w4, bits);
+  return r;
+}
+
+// How elements fall into packs: [0, head) single elements up to the first 16-byte
+// boundary of the destinations, then `packs` packs, then the rest element by element. With
+// destinations at different phases there are no packs. `off`: the first byte in every destination.
+struct PackSplit { uint64_t head, packs; };
+__device__ __forceinline__ PackSplit split_packs(void* const* dst, int ndst, uint64_t off, uint64_t count, uint32_t esz) {
+  const uint32_t phase = (uint32_t)((uintptr_t)dst[0] + off) & 15u;
+  bool same = true;
+  for (int d = 1; d < ndst; d++) same &= ((uint32_t)((uintptr_t)dst[d] + off) & 15u) == phase;
+  PackSplit s;
+  s.head = same ? ((16u - phase) & 15u) / esz : count;
+  if (s.head > count) s.head = count;
+  s.packs = (count - s.head) / (16u / esz);
+  return s;
+}
+
 #ifdef MCCS_UNTYPED_KERNELS
 __global__ void __launch_bounds__(kMaxThreads) ag_ring_kernel(const __grid_constant__ CollArgs a) {
   const int rank = a.emulated ? (int)blockIdx.y : a.rank;
@@ -605,7 +644,7 @@ __global__ void __launch_bounds__(kMaxThreads) local_copy_kernel(const __grid_co
   const uint64_t bytes = a.count;  // the launcher converts elements to bytes
   if (in != out) {
     uint64_t done = 0;
-    if ((((uint64_t)in | (uint64_t)out) & 15u) == 0) {
+    if ((((uint64_t)in | (uint64_t)out) & 15u) == 0) {   // (elsewhere local_copy_ragged_kernel is the faster one)
       const uint64_t nv = bytes / 16;
       const uint64_t tile = (uint64_t)blockDim.x * kCopyUnroll;
       const Raw<16>* src = (const Raw<16>*)in;
@@ -628,6 +667,39 @@ __global__ void __launch_bounds__(kMaxThreads) local_copy_kernel(const __grid_co
     for (uint64_t i = done + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < bytes; i += stride) out[i] = in[i];
   }
   if (a.pad[rank] != nullptr) finish<true>(a, rank);   // no completion word for callers without a communicator
+}
+
+// The same for buffers that are not both 16-byte aligned: the packs are aligned in the output, the
+// input's bytes are shifted into place (one element at a time this ran at 32 GB/s).
+__global__ void __launch_bounds__(kMaxThreads) local_copy_ragged_kernel(const __grid_constant__ CollArgs a) {
+  wait_for_previous_kernel();
+  trace_begin(a, a.rank);
+  const char* in = (const char*)a.send[a.rank];
+  char* out = (char*)a.recv[a.rank];
+  if (in != out) {
+    const PackSplit ps = split_packs(a.recv + a.rank, 1, 0, a.count, 1);
+    const uint32_t shift = (uint32_t)((uintptr_t)in + ps.head) & 15u;
+    const uint64_t tile = (uint64_t)blockDim.x * kCopyUnroll;
+    for (uint64_t base = (uint64_t)blockIdx.x * tile; base < ps.packs; base += (uint64_t)gridDim.x * tile) {
+      Raw<16> v[kCopyUnroll];
+#pragma unroll
+      for (int u = 0; u < kCopyUnroll; u++) {
+        const uint64_t i = base + threadIdx.x + (uint64_t)u * blockDim.x;
+        if (i < ps.packs) v[u] = ld_shifted(in + ps.head + i * 16, shift);
+      }
+#pragma unroll
+      for (int u = 0; u < kCopyUnroll; u++) {
+        const uint64_t i = base + threadIdx.x + (uint64_t)u * blockDim.x;
+        if (i < ps.packs) st_local<16>(out + ps.head + i * 16, v[u]);
+      }
+    }
+    const uint64_t single = a.count - ps.packs * 16;   // fewer than 32: CTA 0 has a thread for each
+    if (blockIdx.x == 0 && threadIdx.x < single) {
+      const uint64_t k = threadIdx.x < ps.head ? threadIdx.x : threadIdx.x + ps.packs * 16;
+      out[k] = in[k];
+    }
+  }
+  if (a.pad[a.rank] != nullptr) finish<true>(a, a.rank);
 }
 
 #endif  // MCCS_UNTYPED_KERNELS

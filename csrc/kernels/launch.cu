@@ -15,6 +15,7 @@ const void* mccs_kfn_f32(int, int);
 const void* mccs_kfn_f64(int, int);
 const void* mccs_kfn_bf16(int, int);
 const void* mccs_kfn_untyped(int);
+const void* mccs_kfn_local_copy_ragged();
 const void* mccs_kfn_one_gpu_i8(int, int, int);
 const void* mccs_kfn_one_gpu_u8(int, int, int);
 const void* mccs_kfn_one_gpu_i32(int, int, int);
@@ -225,6 +226,7 @@ cudaError_t launch_collective(int kind, const CollArgs& args, LaunchDims dims, v
   dim3 grid((unsigned)dims.ctas, a.emulated ? (unsigned)a.nranks : 1u, 1u);
   dim3 block((unsigned)dims.threads, 1u, 1u);
   void* params[] = {(void*)&a};
+  if (a.variant == kLocalCopy && (((uint64_t)a.send[a.rank] | (uint64_t)a.recv[a.rank]) & 15u) != 0) fn = mccs_kfn_local_copy_ragged();
   if (a.variant == kLocalCopy) return launch_local(fn, grid, block, params, stream);
   if (a.emulated && a.nranks > 1) {
     // All ranks' CTAs wait on one another, so they must be resident together.

@@ -26,43 +26,6 @@
 namespace mccs {
 namespace dev {
 
-// The 16 bytes at `p`, which lies `shift` bytes (0..15) behind a 16-byte boundary. `shift` is
-// the same in the whole grid. Both aligned packs that are read hold at least one byte of the
-// 16, so neither lies outside the page of the data.
-__device__ __forceinline__ Raw<16> ld_shifted(const char* p, uint32_t shift) {
-  const char* q = p - shift;
-  const Raw<16> lo = ld_local<16>(q);
-  if (shift == 0) return lo;
-  const Raw<16> hi = ld_local<16>(q + 16);
-  uint32_t w0 = lo.x, w1 = lo.y, w2 = lo.z, w3 = lo.w, w4 = hi.x;
-  if (shift & 8u) { w0 = lo.z; w1 = lo.w; w2 = hi.x; w3 = hi.y; w4 = hi.z; }
-  uint32_t w5 = (shift & 8u) ? hi.w : hi.y;
-  if (shift & 4u) { w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; }
-  const uint32_t bits = (shift & 3u) * 8u;
-  Raw<16> r;
-  r.x = funnel_right(w0, w1, bits);
-  r.y = funnel_right(w1, w2, bits);
-  r.z = funnel_right(w2, w3, bits);
-  r.w = funnel_right(w3, w4, bits);
-  return r;
-}
-
-// How one group's elements fall into packs: [0, head) single elements up to the first 16-byte
-// boundary of the destinations, then `packs` packs, then the rest element by element. With
-// destinations at different phases there are no packs. `off`: the group's first byte in every
-// destination.
-struct PackSplit { uint64_t head, packs; };
-__device__ __forceinline__ PackSplit split_packs(void* const* dst, int ndst, uint64_t off, uint64_t count, uint32_t esz) {
-  const uint32_t phase = (uint32_t)((uintptr_t)dst[0] + off) & 15u;
-  bool same = true;
-  for (int d = 1; d < ndst; d++) same &= ((uint32_t)((uintptr_t)dst[d] + off) & 15u) == phase;
-  PackSplit s;
-  s.head = same ? ((16u - phase) & 15u) / esz : count;
-  if (s.head > count) s.head = count;
-  s.packs = (count - s.head) / (16u / esz);
-  return s;
-}
-
 // Completion word of the launch, as finish() in collectives.cuh, for the whole grid at once.
 // Everything the kernel wrote is memory of this GPU, so ordering the CTAs' stores at GPU scope
 // before the count is enough; the word itself is a plain store to host memory behind the last

@@ -18,6 +18,8 @@ extern "C" const void* mccs_kfn_untyped(int variant) {
   return nullptr;
 }
 
+extern "C" const void* mccs_kfn_local_copy_ragged() { return (const void*)&local_copy_ragged_kernel; }
+
 extern "C" const void* mccs_kfn_group_gather(int nranks, int ragged) {
   if (nranks <= 2) return ragged ? (const void*)&group_gather_ragged_kernel<2> : (const void*)&group_gather_kernel<2>;
   if (nranks <= 4) return ragged ? (const void*)&group_gather_ragged_kernel<4> : (const void*)&group_gather_kernel<4>;

@@ -4,38 +4,42 @@
 // A collective on a small message costs the GPU a few microseconds; written in Python over ctypes
 // its call alone cost four (keyword handling 0.3, looking up the current stream 1.3, the capture
 // check 0.3, argument objects and the ctypes call 1.5), which n ranks driven by one thread pay n
-// times. Here it is 0.5: the tensor's three properties, one dictionary look-up each for
-// type, operator and variant, and the C call with the interpreter lock released.
+// times. Here it is under half a microsecond: the tensors are read through torch's C++ interface,
+// one dictionary look-up each for operator and variant, and the C call with the interpreter lock
+// released.
 //
 // The C API's functions arrive as addresses (`bind`), so that this module always talks to the
-// libmccs.so the package has loaded and links against nothing.
+// libmccs.so the package has loaded.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <c10/cuda/CUDAStream.h>
 #include <cuda.h>
 #include <dlfcn.h>
 #include <stdint.h>
+#include <torch/csrc/autograd/python_variable.h>
 
 #include "../include/mccs.h"
+#include "../include/mccs_noalloc.h"
 
 namespace {
 
 decltype(&mccsAllReduceEx) g_all_reduce;
 decltype(&mccsAllGatherEx) g_all_gather;
 decltype(&mccsReduceScatterEx) g_reduce_scatter;
+decltype(&mccsCommSelfCopy) g_self_copy;
+decltype(&mccsCommTakesAnyMemory) g_takes_any_memory;
 decltype(&mccsGroupStart) g_group_start;
 decltype(&mccsGroupEnd) g_group_end;
 
 // Owned for the life of the process.
-PyObject* g_tensor_type;      // torch.Tensor
 PyObject* g_dtypes;           // torch.dtype -> mccsDataType_t
 PyObject* g_ops;              // operator name -> mccsRedOp_t
 PyObject* g_algos;            // variant name -> mccsAlgo_t
 PyObject* g_error;            // MccsError(code, what)
 PyObject* g_buffer_type;      // Buffer
-PyObject* g_current_stream;   // device index -> raw handle of torch's current stream; None without CUDA
 PyObject* g_capturing;        // () -> is the current stream of the current device capturing; None without CUDA
-PyObject *s_data_ptr, *s_numel, *s_element_size, *s_dtype, *s_lower, *s_cuda_stream, *s_ptr;
+PyObject *s_lower, *s_cuda_stream, *s_ptr;
 
 // The driver calls of the capture check, when libcuda is there.
 decltype(&cuStreamIsCapturing) g_is_capturing;
@@ -46,9 +50,33 @@ struct Calls {
   mccsComm_t comm;
   int device;
   int cuda;     // the daemon's backend is CUDA
+  int any_memory;   // mccsCommTakesAnyMemory
 };
 
-bool is_tensor(PyObject* o) { return PyObject_TypeCheck(o, (PyTypeObject*)g_tensor_type); }
+const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// mccsDataType_t of a tensor; KeyError with the type, as the dictionary raises it, for another one.
+bool type_code(const at::Tensor& t, PyObject* of, int* out) {
+  switch (t.scalar_type()) {
+    case at::kChar: *out = mccsInt8; return true;
+    case at::kByte: *out = mccsUint8; return true;
+    case at::kInt: *out = mccsInt32; return true;
+    case at::kUInt32: *out = mccsUint32; return true;
+    case at::kLong: *out = mccsInt64; return true;
+    case at::kUInt64: *out = mccsUint64; return true;
+    case at::kHalf: *out = mccsFloat16; return true;
+    case at::kFloat: *out = mccsFloat32; return true;
+    case at::kDouble: *out = mccsFloat64; return true;
+    case at::kBFloat16: *out = mccsBfloat16; return true;
+    default: break;
+  }
+  PyObject* d = PyObject_GetAttrString(of, "dtype");
+  if (d) {
+    PyErr_SetObject(PyExc_KeyError, d);
+    Py_DECREF(d);
+  }
+  return false;
+}
 
 bool to_u64(PyObject* o, uint64_t* out) {   // steals nothing
   PyObject* i = PyNumber_Index(o);
@@ -62,17 +90,9 @@ bool to_u64(PyObject* o, uint64_t* out) {   // steals nothing
   return !PyErr_Occurred();
 }
 
-bool method_u64(PyObject* o, PyObject* name, uint64_t* out) {
-  PyObject* r = PyObject_CallMethodNoArgs(o, name);
-  if (!r) return false;
-  *out = (uint64_t)PyLong_AsUnsignedLongLongMask(r);
-  Py_DECREF(r);
-  return !PyErr_Occurred();
-}
-
 // Address of a tensor, a Buffer or a raw pointer.
 bool address(PyObject* o, uint64_t* out) {
-  if (is_tensor(o)) return method_u64(o, s_data_ptr, out);
+  if (const at::Tensor* t = tensor(o)) { *out = (uint64_t)t->data_ptr(); return true; }
   if (PyObject_TypeCheck(o, (PyTypeObject*)g_buffer_type)) {
     PyObject* p = PyObject_GetAttr(o, s_ptr);
     if (!p) return false;
@@ -122,12 +142,7 @@ PyObject* raise(int code, const char* what) {
 bool resolve_stream(Calls* self, PyObject* stream, uint64_t* out) {
   *out = 0;
   if (self->cuda) {
-    PyObject* dev = PyLong_FromLong(self->device);
-    PyObject* cur = dev ? PyObject_CallOneArg(g_current_stream, dev) : nullptr;
-    Py_XDECREF(dev);
-    if (!cur) return false;
-    const uint64_t current = (uint64_t)PyLong_AsUnsignedLongLongMask(cur);
-    Py_DECREF(cur);
+    const uint64_t current = (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
     bool capturing = false, known = false;
     CUdevice now = -1;
     if (g_is_capturing && g_ctx_device && g_ctx_device(&now) == CUDA_SUCCESS && (int)now == self->device) {
@@ -191,15 +206,9 @@ PyObject* reducing(Calls* self, PyObject* const* args, Py_ssize_t nargs, PyObjec
   bool have_count = given(a[2]), have_dtype = given(a[3]);
   if (have_count && !to_u64(a[2], &count)) return nullptr;
   if (have_dtype && !lookup(g_dtypes, a[3], &dtype)) return nullptr;
-  if (is_tensor(shape)) {
-    if (!have_count && !method_u64(shape, s_numel, &count)) return nullptr;
-    if (!have_dtype) {
-      PyObject* d = PyObject_GetAttr(shape, s_dtype);
-      if (!d) return nullptr;
-      const bool ok = lookup(g_dtypes, d, &dtype);
-      Py_DECREF(d);
-      if (!ok) return nullptr;
-    }
+  if (const at::Tensor* t = tensor(shape)) {
+    if (!have_count) count = (uint64_t)t->numel();
+    if (!have_dtype && !type_code(*t, shape, &dtype)) return nullptr;
   } else if (!have_count || !have_dtype) {
     PyErr_SetString(PyExc_ValueError, "dtype and count are needed for raw pointers");
     return nullptr;
@@ -227,15 +236,15 @@ PyObject* reducing(Calls* self, PyObject* const* args, Py_ssize_t nargs, PyObjec
   Py_RETURN_NONE;
 }
 
-PyObject* calls_all_reduce(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+PyObject* all_reduce(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
   return reducing((Calls*)self, args, nargs, kwnames, "all_reduce", "mccsAllReduce", false);
 }
 
-PyObject* calls_reduce_scatter(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+PyObject* reduce_scatter(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
   return reducing((Calls*)self, args, nargs, kwnames, "reduce_scatter", "mccsReduceScatter", true);
 }
 
-PyObject* calls_all_gather(PyObject* self_, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+PyObject* all_gather(PyObject* self_, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
   static const char* const names[] = {"send", "recv", "nbytes", "algo", "stream"};
   Calls* self = (Calls*)self_;
   PyObject* a[5] = {nullptr};
@@ -243,10 +252,8 @@ PyObject* calls_all_gather(PyObject* self_, PyObject* const* args, Py_ssize_t na
   uint64_t nbytes = 0, send_va, recv_va, stream;
   if (given(a[2])) {
     if (!to_u64(a[2], &nbytes)) return nullptr;
-  } else if (is_tensor(a[0])) {
-    uint64_t n = 0, esz = 0;
-    if (!method_u64(a[0], s_numel, &n) || !method_u64(a[0], s_element_size, &esz)) return nullptr;
-    nbytes = n * esz;
+  } else if (const at::Tensor* t = tensor(a[0])) {
+    nbytes = (uint64_t)t->numel() * (uint64_t)t->element_size();
   } else {
     PyErr_SetString(PyExc_ValueError, "nbytes is needed for raw pointers");
     return nullptr;
@@ -264,26 +271,72 @@ PyObject* calls_all_gather(PyObject* self_, PyObject* const* args, Py_ssize_t na
   Py_RETURN_NONE;
 }
 
-PyObject* calls_attach(PyObject* self_, PyObject* args) {
+// self_copy(send, recv, stream) -> bool. Any collective of a communicator of one rank whose tensors
+// are plain memory of its GPU: one copy kernel on them where they are. False when that does not apply
+// (more ranks, other devices, other layouts, differing types) and the caller has to stage.
+PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
+  Calls* self = (Calls*)self_;
+  if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "self_copy(send, recv, stream)"); return nullptr; }
+  const at::Tensor* in = self->any_memory ? tensor(args[0]) : nullptr;
+  const at::Tensor* out = in ? tensor(args[1]) : nullptr;
+  if (!out || !in->is_cuda() || !out->is_cuda() || in->get_device() != self->device || out->get_device() != self->device ||
+      in->scalar_type() != out->scalar_type() || in->numel() != out->numel() || in->numel() == 0 || !in->is_contiguous() || !out->is_contiguous())
+    Py_RETURN_FALSE;
+  uint64_t stream;
+  if (!resolve_stream(self, args[2], &stream)) return nullptr;
+  const void* const from = in->data_ptr();
+  void* const to = out->data_ptr();
+  const size_t bytes = (size_t)in->numel() * (size_t)in->element_size();
+  mccsResult_t rc;
+  const mccsComm_t comm = self->comm;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_self_copy(comm, from, to, bytes, (mccsStream_t)stream);
+  Py_END_ALLOW_THREADS
+  if (rc == mccsUnsupported) Py_RETURN_FALSE;
+  if (rc != mccsSuccess) return raise(rc, "mccsCommSelfCopy");
+  Py_RETURN_TRUE;
+}
+
+PyObject* attach(PyObject* self_, PyObject* args) {
   Calls* self = (Calls*)self_;
   unsigned long long h = 0;
   if (!PyArg_ParseTuple(args, "Kii", &h, &self->device, &self->cuda)) return nullptr;
   self->comm = (mccsComm_t)h;
+  self->any_memory = self->comm ? g_takes_any_memory(self->comm) : 0;
   Py_RETURN_NONE;
 }
 
+// A tensor without storage throws when it is asked for its address: a Python error, not the end of
+// the process.
+template <typename... Args> PyObject* caught(PyObject* (*fn)(Args...), Args... args) {
+  try {
+    return fn(args...);
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {
+    PyErr_SetString(PyExc_RuntimeError, "unknown C++ exception");
+  }
+  return nullptr;
+}
+template <PyObject* (*fn)(PyObject*, PyObject* const*, Py_ssize_t, PyObject*)>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n, PyObject* kw) { return caught(fn, self, args, n, kw); }
+template <PyObject* (*fn)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) { return caught(fn, self, args, n); }
+
 PyMethodDef calls_methods[] = {
-    {"all_reduce", (PyCFunction)(void (*)(void))calls_all_reduce, METH_FASTCALL | METH_KEYWORDS,
+    {"all_reduce", (PyCFunction)(void (*)(void))(_PyCFunctionFastWithKeywords)guarded<all_reduce>, METH_FASTCALL | METH_KEYWORDS,
      "all_reduce(send, recv=None, *, count=None, dtype=None, op='sum', scale=1.0, algo='auto', stream=None)\n"
      "AllReduce ``count`` elements; in place when ``recv`` is None."},
-    {"all_gather", (PyCFunction)(void (*)(void))calls_all_gather, METH_FASTCALL | METH_KEYWORDS,
+    {"all_gather", (PyCFunction)(void (*)(void))(_PyCFunctionFastWithKeywords)guarded<all_gather>, METH_FASTCALL | METH_KEYWORDS,
      "all_gather(send, recv, *, nbytes=None, algo='auto', stream=None)\n"
      "AllGather ``nbytes`` per rank into ``recv`` (``nranks * nbytes`` bytes)."},
-    {"reduce_scatter", (PyCFunction)(void (*)(void))calls_reduce_scatter, METH_FASTCALL | METH_KEYWORDS,
+    {"reduce_scatter", (PyCFunction)(void (*)(void))(_PyCFunctionFastWithKeywords)guarded<reduce_scatter>, METH_FASTCALL | METH_KEYWORDS,
      "reduce_scatter(send, recv, *, count=None, dtype=None, op='sum', scale=1.0, algo='auto', stream=None)\n"
      "ReduceScatter: ``send`` holds ``nranks * count`` elements, ``recv`` receives the reduction of block ``rank``\n"
      "(``count`` elements). In place when ``recv`` is the rank's own block of ``send``. The reference has no such call."},
-    {"_attach", calls_attach, METH_VARARGS, "_attach(handle, device, is_cuda): the communicator the calls go to (handle 0: none)"},
+    {"self_copy", (PyCFunction)(void (*)(void))(_PyCFunctionFast)guarded<self_copy>, METH_FASTCALL,
+     "self_copy(send, recv, stream) -> bool: a one-rank collective on ordinary CUDA tensors, in place of staging"},
+    {"_attach", attach, METH_VARARGS, "_attach(handle, device, is_cuda): the communicator the calls go to (handle 0: none)"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyTypeObject calls_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
@@ -304,25 +357,83 @@ PyObject* module_group_end(PyObject*, PyObject* quiet) {
   Py_RETURN_NONE;
 }
 
-// bind(functions, tensor type, Buffer, dtypes, ops, algos, MccsError, current stream, capturing)
+// local_all_reduce(address of mccsLocalAllReduceNoAlloc, inputs, outputs, stream) -> its return value,
+// or None when the tensors' device is not the current one (the caller makes it so and comes back).
+PyObject* local_all_reduce(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 4) { PyErr_SetString(PyExc_TypeError, "local_all_reduce(function, inputs, outputs, stream)"); return nullptr; }
+  const auto fn = (decltype(&mccsLocalAllReduceNoAlloc))PyLong_AsUnsignedLongLong(args[0]);
+  if (PyErr_Occurred()) return nullptr;
+  PyObject* seq[2] = {PySequence_Fast(args[1], "inputs"), nullptr};
+  if (seq[0]) seq[1] = PySequence_Fast(args[2], "outputs");
+  if (!seq[1]) { Py_XDECREF(seq[0]); return nullptr; }
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq[0]);
+  const char* bad = nullptr;
+  void* at[2][MCCS_NOALLOC_MAX_RANKS];
+  int dtype = 0, device = -1;
+  int64_t count = 0;
+  if (n == 0) bad = "no tensors";
+  else if (n != PySequence_Fast_GET_SIZE(seq[1]) || n > MCCS_NOALLOC_MAX_RANKS) bad = "need as many outputs as inputs, at most 8";
+  const at::Tensor* first = nullptr;
+  for (int side = 0; side < 2 && !bad; side++)
+    for (Py_ssize_t i = 0; i < n && !bad; i++) {
+      const at::Tensor* t = tensor(PySequence_Fast_GET_ITEM(seq[side], i));
+      if (!first) first = t;
+      if (!t || !t->is_cuda() || t->get_device() != first->get_device() || t->scalar_type() != first->scalar_type() || t->numel() != first->numel() ||
+          !t->is_contiguous())
+        bad = "tensors must be contiguous CUDA tensors of one device, dtype and size";
+      else
+        at[side][i] = t->data_ptr();
+    }
+  if (!bad) {
+    device = (int)first->get_device();
+    count = first->numel();
+    switch (first->scalar_type()) {
+      case at::kFloat: dtype = mccsFloat32; break;
+      case at::kHalf: dtype = mccsFloat16; break;
+      case at::kBFloat16: dtype = mccsBfloat16; break;
+      default: bad = "float32, float16 or bfloat16 only";
+    }
+  }
+  Py_DECREF(seq[0]);
+  Py_DECREF(seq[1]);
+  if (bad) { PyErr_SetString(PyExc_ValueError, bad); return nullptr; }
+  CUdevice now = -1;
+  if (!g_ctx_device || g_ctx_device(&now) != CUDA_SUCCESS || (int)now != device) Py_RETURN_NONE;
+  uint64_t stream = 0;
+  if (args[3] == Py_None) {
+    stream = (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+  } else {
+    PyObject* h = PyObject_GetAttr(args[3], s_cuda_stream);
+    const bool ok = h && to_u64(h, &stream);
+    Py_XDECREF(h);
+    if (!ok) return nullptr;
+  }
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = fn(at[0], at[1], (int)n, (size_t)count, dtype, (void*)stream);
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+}
+
+// bind(functions, Buffer, dtypes, ops, algos, MccsError, capturing)
 PyObject* module_bind(PyObject*, PyObject* args) {
-  unsigned long long ar, ag, rs, gs, ge;
-  PyObject *tensor, *buffer, *dtypes, *ops, *algos, *error, *current, *capturing;
-  if (!PyArg_ParseTuple(args, "(KKKKK)OOO!O!O!OOO", &ar, &ag, &rs, &gs, &ge, &tensor, &buffer, &PyDict_Type, &dtypes, &PyDict_Type, &ops,
-                        &PyDict_Type, &algos, &error, &current, &capturing))
+  unsigned long long ar, ag, rs, gs, ge, sc, am;
+  PyObject *buffer, *dtypes, *ops, *algos, *error, *capturing;
+  if (!PyArg_ParseTuple(args, "(KKKKKKK)OO!O!O!OO", &ar, &ag, &rs, &gs, &ge, &sc, &am, &buffer, &PyDict_Type, &dtypes, &PyDict_Type, &ops,
+                        &PyDict_Type, &algos, &error, &capturing))
     return nullptr;
   g_all_reduce = (decltype(g_all_reduce))ar;
   g_all_gather = (decltype(g_all_gather))ag;
   g_reduce_scatter = (decltype(g_reduce_scatter))rs;
   g_group_start = (decltype(g_group_start))gs;
   g_group_end = (decltype(g_group_end))ge;
-  g_tensor_type = Py_NewRef(tensor);
+  g_self_copy = (decltype(g_self_copy))sc;
+  g_takes_any_memory = (decltype(g_takes_any_memory))am;
   g_buffer_type = Py_NewRef(buffer);
   g_dtypes = Py_NewRef(dtypes);
   g_ops = Py_NewRef(ops);
   g_algos = Py_NewRef(algos);
   g_error = Py_NewRef(error);
-  g_current_stream = Py_NewRef(current);
   g_capturing = Py_NewRef(capturing);
   if (void* lib = dlopen("libcuda.so.1", RTLD_NOW | RTLD_LOCAL)) {
     g_is_capturing = (decltype(g_is_capturing))dlsym(lib, "cuStreamIsCapturing");
@@ -334,6 +445,7 @@ PyObject* module_bind(PyObject*, PyObject* args) {
 PyMethodDef module_methods[] = {{"bind", module_bind, METH_VARARGS, nullptr},
                                 {"group_start", module_group_start, METH_NOARGS, nullptr},
                                 {"group_end", module_group_end, METH_O, nullptr},
+                                {"local_all_reduce", (PyCFunction)(void (*)(void))(_PyCFunctionFast)guarded<local_all_reduce>, METH_FASTCALL, nullptr},
                                 {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_calls", "Collective calls of mccs_b200.", -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
@@ -346,10 +458,6 @@ PyMODINIT_FUNC PyInit__calls(void) {
   calls_type.tp_methods = calls_methods;
   calls_type.tp_new = PyType_GenericNew;
   if (PyType_Ready(&calls_type) < 0) return nullptr;
-  s_data_ptr = PyUnicode_InternFromString("data_ptr");
-  s_numel = PyUnicode_InternFromString("numel");
-  s_element_size = PyUnicode_InternFromString("element_size");
-  s_dtype = PyUnicode_InternFromString("dtype");
   s_lower = PyUnicode_InternFromString("lower");
   s_cuda_stream = PyUnicode_InternFromString("cuda_stream");
   s_ptr = PyUnicode_InternFromString("ptr");

@@ -827,6 +827,7 @@ mccsResult_t submit_memops(mccsComm* comm, proto::WorkRequest& wr, mccsStream_t 
 // Address, in this process, of byte `off` of allocation `mem_id`: one of the caller's own
 // allocations, or a peer's, mapped on first use (client-side launch only).
 mccsResult_t resolve_mem(std::unique_lock<std::mutex>& g, mccsComm* comm, uint64_t mem_id, uint64_t off, uint64_t* out) {
+  if (mem_id == 0 && comm->nranks == 1) { *out = off; return mccsSuccess; }   // proto::kWrExternal
   auto own = g_ctx.mem_base_by_id.find(mem_id);
   if (own != g_ctx.mem_base_by_id.end()) { *out = own->second + off; return mccsSuccess; }
   auto it = comm->peer_mem.find(mem_id);
@@ -1181,15 +1182,20 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
   {
     std::unique_lock<std::mutex> g(g_ctx.mu);
     if (!g_ctx.connected) return mccsNotConnected;
-    const MemRec* sm = find_mem_locked(send);
-    const MemRec* rm = find_mem_locked(recv);
-    if (!sm || !rm) {
-      LOG_ERROR("collective buffers must come from mccsMalloc (send %p, recv %p)", send, recv);
-      return mccsInvalidArgument;
+    if (wr.flags & proto::kWrExternal) {
+      wr.send_off = (uint64_t)send;
+      wr.recv_off = (uint64_t)recv;
+    } else {
+      const MemRec* sm = find_mem_locked(send);
+      const MemRec* rm = find_mem_locked(recv);
+      if (!sm || !rm) {
+        LOG_ERROR("collective buffers must come from mccsMalloc (send %p, recv %p)", send, recv);
+        return mccsInvalidArgument;
+      }
+      wr.send_mem = sm->mem_id; wr.send_off = (uint64_t)send - sm->base;
+      wr.recv_mem = rm->mem_id; wr.recv_off = (uint64_t)recv - rm->base;
+      if (wr.send_off + send_bytes > sm->size || wr.recv_off + recv_bytes > rm->size) return mccsInvalidArgument;
     }
-    wr.send_mem = sm->mem_id; wr.send_off = (uint64_t)send - sm->base;
-    wr.recv_mem = rm->mem_id; wr.recv_off = (uint64_t)recv - rm->base;
-    if (wr.send_off + send_bytes > sm->size || wr.recv_off + recv_bytes > rm->size) return mccsInvalidArgument;
     if (!comm->sync_base && !comm->client_launch && !on_caller_stream) {
       mccsResult_t r = register_stream_locked(g, comm->device, stream, &srec);
       if (r != mccsSuccess) return r;
@@ -1725,6 +1731,24 @@ mccsResult_t mccsAllGatherEx(mccsComm_t comm, const void* send, void* recv, size
 
 mccsResult_t mccsAllGather(mccsComm_t comm, const void* send, void* recv, size_t bytes, mccsStream_t stream) {
   return mccsAllGatherEx(comm, send, recv, bytes, mccsAlgoAuto, stream);
+}
+
+int mccsCommTakesAnyMemory(mccsComm_t comm) {
+  return comm && comm->nranks == 1 && g_ctx.backend == proto::kBackendCuda && (comm->client_launch || comm->caller_streams) ? 1 : 0;
+}
+
+mccsResult_t mccsCommSelfCopy(mccsComm_t comm, const void* send, void* recv, size_t bytes, mccsStream_t stream) {
+  if (!mccsCommTakesAnyMemory(comm) || (comm->caller_streams && (comm->deferred_wait || stream == (mccsStream_t)CU_STREAM_PER_THREAD)))
+    return mccsUnsupported;
+  if (bytes > (1ull << 44) || !send || !recv) return mccsInvalidArgument;
+  proto::WorkRequest wr;
+  memset(&wr, 0, sizeof wr);
+  wr.kind = kAllGather;
+  wr.dtype = kUint8;
+  wr.count = bytes;
+  wr.scale = 1.0f;
+  wr.flags = proto::kWrExternal;
+  return submit(comm, wr, send, recv, bytes, bytes, stream);
 }
 
 mccsResult_t mccsCommSetDeferredWait(mccsComm_t comm, int on) {

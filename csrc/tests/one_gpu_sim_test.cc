@@ -147,6 +147,33 @@ void gather_case(int n, size_t count, const std::vector<size_t>& send_off, const
   if (!good) { g_failed++; fprintf(stderr, "FAILED: gather n %d count %zu in_place %d ragged %d ctas %d\n", n, count, in_place, ragged, ctas); }
 }
 
+void copy_case(size_t count, size_t send_off, size_t recv_off, int ctas, int threads) {
+  Block in(count, send_off), out(count, recv_off);
+  for (size_t i = 0; i < count; i++) in.p()[i] = (uint8_t)(i * 11 + 3);
+  SignalPad* pad = (SignalPad*)aligned_alloc(128, sizeof(SignalPad));
+  memset(pad, 0, sizeof *pad);
+  StatusBlock status;
+  memset(&status, 0, sizeof status);
+  CollArgs a;
+  memset(&a, 0, sizeof a);
+  a.nranks = 1;
+  a.count = count;
+  a.seq = 5;
+  a.send[0] = in.p(); a.recv[0] = out.p();
+  a.pad[0] = pad; a.status[0] = &status;
+  std::vector<std::thread> pool;
+  sim::Dim3 grid;
+  grid.x = (unsigned)ctas;
+  sim::launch(local_copy_ragged_kernel, grid, (unsigned)threads, a, &pool);
+  sim::join_all(&pool);
+  g_cases++;
+  if (memcmp(in.p(), out.p(), count) != 0 || !out.guards_intact() || status.done_seq != 5 || pad->pad_[kPadCtaCounter] != 0) {
+    g_failed++;
+    fprintf(stderr, "FAILED: ragged copy of %zu bytes, phases %zu -> %zu, %d CTAs\n", count, send_off, recv_off, ctas);
+  }
+  free(pad);
+}
+
 template <typename T>
 void type_cases() {
   const size_t per = 16 / sizeof(T);
@@ -189,6 +216,9 @@ int main() {
       gather_case(n, count, mixed, same, false, 2, 64);
       gather_case(n, count, zero, mixed, true, 2, 32);
     }
+  for (size_t count : {(size_t)1, (size_t)15, (size_t)16, (size_t)31, (size_t)2048, (size_t)2049, (size_t)5003})
+    for (size_t so = 0; so < 16; so++)
+      for (size_t ro : {(size_t)0, (size_t)1, (size_t)8, (size_t)15}) copy_case(count, so, ro, 2, 32);
   printf("one_gpu_sim_test: %d cases, %d failed\n", g_cases, g_failed);
   return g_failed ? 1 : 0;
 }

@@ -144,9 +144,10 @@ def calls():
         loader.exec_module(mod)
         lib = shim()
         mod.bind(tuple(ctypes.cast(getattr(lib, f), c_void_p).value for f in
-                       ("mccsAllReduceEx", "mccsAllGatherEx", "mccsReduceScatterEx", "mccsGroupStart", "mccsGroupEnd")),
-                 torch.Tensor, client.Buffer, client.DTYPES, client.OPS, client.ALGOS, MccsError,
-                 getattr(torch._C, "_cuda_getCurrentRawStream", None), torch.cuda.is_current_stream_capturing)
+                       ("mccsAllReduceEx", "mccsAllGatherEx", "mccsReduceScatterEx", "mccsGroupStart", "mccsGroupEnd", "mccsCommSelfCopy",
+                        "mccsCommTakesAnyMemory")),
+                 client.Buffer, client.DTYPES, client.OPS, client.ALGOS, MccsError,
+                 torch.cuda.is_current_stream_capturing)
         _calls = mod
     return _calls
 

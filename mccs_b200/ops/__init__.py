@@ -24,7 +24,9 @@ from typing import Optional, Sequence
 import torch
 
 from .. import _lib
-from ..client import ALGOS, DTYPES, Buffer, Communicator, backend
+from ..client import ALGOS, DTYPES, OPS, Buffer, Communicator, backend
+
+_PREMULSUM = OPS["premulsum"]
 
 VARIANTS = {
     "auto": "the planner's choice from the measured size -> (variant, CTAs) table",
@@ -98,10 +100,13 @@ def all_reduce(comm: Communicator, send: torch.Tensor, recv: Optional[torch.Tens
     Tensors in service memory (:class:`mccs_b200.Buffer`) are used where they are; any other
     tensor (ordinary CUDA memory, unsupported element type such as bool, non-contiguous) is
     staged through the communicator's arena: one copy in, the collective in place, one copy
-    out, all on the caller's stream. Returns the output tensor; like a kernel launch, the call
+    out, all on the caller's stream (a communicator of one rank copies from tensor to tensor
+    instead, wherever they are on its GPU). Returns the output tensor; like a kernel launch, the call
     returns before the result exists."""
     out = send if recv is None else recv
     if send.numel() == 0:
+        return out
+    if comm.nranks == 1 and OPS[op.lower()] != _PREMULSUM and comm._calls.self_copy(send, out, stream):
         return out
     if usable_in_place(send) and (recv is None or usable_in_place(recv)):
         comm.all_reduce(send, recv, op=op, scale=scale, algo=algo, stream=stream)
@@ -124,6 +129,8 @@ def all_gather(comm: Communicator, send: torch.Tensor, recv: torch.Tensor, *, al
     :func:`all_reduce` when a tensor is not in service memory."""
     nb = send.numel() * send.element_size()
     if nb == 0:
+        return recv
+    if comm.nranks == 1 and comm._calls.self_copy(send, recv, stream):
         return recv
     if usable_in_place(recv) and send.is_contiguous() and in_service_memory(send):
         comm.all_gather(send, recv, nbytes=nb, algo=algo, stream=stream)
@@ -149,6 +156,8 @@ def reduce_scatter(comm: Communicator, send: torch.Tensor, recv: torch.Tensor, *
     Staged like :func:`all_reduce` when a tensor is not in service memory."""
     if recv.numel() == 0:
         return recv
+    if comm.nranks == 1 and OPS[op.lower()] != _PREMULSUM and comm._calls.self_copy(send, recv, stream):
+        return recv
     if usable_in_place(send) and usable_in_place(recv):
         comm.reduce_scatter(send, recv, op=op, scale=scale, algo=algo, stream=stream)
         return recv
@@ -165,38 +174,31 @@ def reduce_scatter(comm: Communicator, send: torch.Tensor, recv: torch.Tensor, *
     return recv
 
 
+_no_alloc_address = 0
+
+
+def _no_alloc_entry() -> int:
+    global _no_alloc_address
+    if not _no_alloc_address:      # raises when the native library is missing: no silent fallback
+        _no_alloc_address = ctypes.cast(_lib.daemon_lib().mccsLocalAllReduceNoAlloc, ctypes.c_void_p).value
+    return _no_alloc_address
+
+
 def local_all_reduce_no_alloc(inputs: Sequence[torch.Tensor], outputs: Optional[Sequence[torch.Tensor]] = None,
                               stream=None) -> Sequence[torch.Tensor]:
     """Sum of up to 8 equally shaped f32 / f16 / bf16 tensors on the CURRENT CUDA device,
-    written to every output (in place when ``outputs`` is None), by the two-shot kernel in
-    one cooperative launch. Allocates nothing, neither here nor in the native code: usable
-    while a memory pool is frozen. Overlapping calls on one device race (they share one
-    scratch array); make the first call on a device outside stream capture."""
-    if not inputs:
-        raise ValueError("no tensors")
-    outs = list(inputs) if outputs is None else list(outputs)
-    first = inputs[0]
-    if len(outs) != len(inputs) or len(inputs) > 8:
-        raise ValueError("need as many outputs as inputs, at most 8")
-    for t in list(inputs) + outs:
-        if not t.is_cuda or t.device != first.device or t.dtype != first.dtype or t.numel() != first.numel() or not t.is_contiguous():
-            raise ValueError("tensors must be contiguous CUDA tensors of one device, dtype and size")
-    if first.dtype not in (torch.float32, torch.float16, torch.bfloat16):
-        raise ValueError("float32, float16 or bfloat16 only")
-    lib = _lib.daemon_lib()          # raises when the native library is missing: no silent fallback
-    fn = lib.mccsLocalAllReduceNoAlloc
-    fn.restype = ctypes.c_int
-    fn.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p), ctypes.c_int, ctypes.c_size_t,
-                   ctypes.c_int, ctypes.c_void_p]
-    n = len(inputs)
-    ins = (ctypes.c_void_p * n)(*[t.data_ptr() for t in inputs])
-    ous = (ctypes.c_void_p * n)(*[t.data_ptr() for t in outs])
-    s = torch.cuda.current_stream(first.device) if stream is None else stream
-    with torch.cuda.device(first.device):
-        rc = fn(ins, ous, n, first.numel(), DTYPES[first.dtype], ctypes.c_void_p(s.cuda_stream))
+    written to every output (in place when ``outputs`` is None), in one pass over memory by one
+    kernel launch. Allocates no device memory, neither here nor in the native code: usable
+    while a memory pool is frozen. Make the first call on a device outside stream capture."""
+    outs = inputs if outputs is None else outputs
+    call = _lib.calls().local_all_reduce      # checks the tensors
+    rc = call(_no_alloc_entry(), inputs, outs, stream)
+    if rc is None:                            # another device is current
+        with torch.cuda.device(inputs[0].device):
+            rc = call(_no_alloc_entry(), inputs, outs, stream)
     if rc != 0:
         raise RuntimeError(f"mccsLocalAllReduceNoAlloc failed with CUDA error {rc}")
-    return outs
+    return list(outs)
 
 
 __all__ = ["VARIANTS", "all_reduce", "all_gather", "reduce_scatter", "in_service_memory", "usable_in_place", "arena",
