@@ -321,7 +321,9 @@ struct alignas(64) DpStatus {
   int32_t first_error;     // Status of the first failed request, 0 = none
   uint32_t last_variant;
   uint32_t last_ctas;
-  uint32_t pad_[11];
+  uint32_t pad_;
+  uint64_t group_closed;   // written by the client: its newest request when it last closed a group
+  uint32_t pad2_[8];
 };
 static_assert(sizeof(DpStatus) == 64, "DpStatus layout is part of the ABI");
 

@@ -81,6 +81,7 @@ struct CollOp {
   uint64_t send_va = 0, recv_va = 0;
   uint64_t send_mem = 0, recv_mem = 0, send_off = 0, recv_off = 0;
   void* user_event = nullptr;
+  bool in_group = false;   // posted inside a group that may bring more requests
   bool on_caller_stream = false;            // ordered against `caller_stream` by the daemon (see proto::CommInitReply)
   void* caller_stream = nullptr;
   uint64_t sync_slot = 0, sync_value = 0;   // mem-op mode (see proto::SyncMode)
@@ -155,7 +156,7 @@ struct RankState {
   proto::WorkRequest pending_wr;
   bool have_pending_wc = false;
   proto::WorkCompletion pending_wc;
-  struct Inflight { uint64_t ticket; uint64_t bytes; };
+  struct Inflight { uint64_t ticket; uint64_t bytes; uint64_t members = 1; };   // members: collectives the launch counts for
   std::deque<Inflight> inflight;       // rank 0 only: admitted, not yet seen finished
   uint64_t traced_ticket = 0;
   std::atomic<uint64_t> last_ticket{0};  // ticket of the newest kernel launched for this rank (rank 0's is read by every proxy of a one-launch group)
@@ -237,6 +238,8 @@ class ProxyEngine : public Engine {
   bool advance(RankState& rs);
   bool plan_slot(Communicator& c, CollSlot& s, uint64_t seq);
   void extend_batch(Communicator& c, CollSlot& head, uint64_t seq, const PlanInput& head_in, uint64_t now);
+  bool wait_for_company(Communicator& c, CollSlot& s, uint64_t seq);
+  void extend_one_gpu(Communicator& c, CollSlot& head, uint64_t seq, const PlanInput& head_in, uint64_t now);
   bool plan_member(Communicator& c, CollSlot& head, CollSlot& m, const PlanInput& head_in, Plan* out);
   void fill_batch_args(Communicator& c, CollSlot& head, uint64_t seq, int rank, BatchArgs* b);
   bool batch_clients_ready(Communicator& c, CollSlot& head, uint64_t seq, int self_rank);

@@ -147,6 +147,7 @@ bool ProxyEngine::post(RankState& rs, const proto::WorkRequest& wr) {
   op.scale = wr.scale;
   op.variant_req = (int)wr.variant;
   op.user_seq = wr.user_seq;
+  op.in_group = (wr.flags & proto::kWrGroupMore) != 0;
   op.on_caller_stream = c.caller_streams && (wr.flags & proto::kWrCallerStream) != 0;
   op.caller_stream = (void*)wr.caller_stream;
   op.sync_slot = wr.sync_slot;
@@ -222,6 +223,27 @@ bool ProxyEngine::followers_still_arriving(Communicator& c, CollSlot& s, uint64_
     const int arrived = m.arrived.load(std::memory_order_acquire);
     if (arrived == 0) return false;              // nobody has posted a follower: nothing to wait for
     if (arrived < c.nranks) return true;         // some have, not all: wait for the rest
+  }
+  return false;
+}
+
+// Ranks that share a GPU: while two launches of the communicator are still ahead on the GPU, a
+// collective of an open group waits for the group's next ones to join its launch (see
+// extend_one_gpu). Nothing is lost by it, the GPU has work for longer than a launch takes to reach
+// it; with fewer ahead it goes at once. The wait ends with the group, with a full launch, and after
+// 50 us in any case (a caller may do something else inside its group).
+bool ProxyEngine::wait_for_company(Communicator& c, CollSlot& s, uint64_t seq) {
+  if (!c.emulated || c.client_launch) return false;
+  const RankState& r0 = *c.ranks[0];
+  if (!r0.dp_status || !r0.status) return false;
+  for (int r = 0; r < c.nranks; r++)
+    if (!s.ops[r].in_group) return false;
+  if (__atomic_load_n(&r0.dp_status->group_closed, __ATOMIC_ACQUIRE) >= s.ops[0].user_seq) return false;
+  if (r0.last_ticket.load(std::memory_order_relaxed) < __atomic_load_n(&r0.status->done_seq, __ATOMIC_ACQUIRE) + 2) return false;
+  if (monotonic_us() - s.t_collected_us.load(std::memory_order_relaxed) > 50) return false;
+  for (int k = 1; k < kMaxBatch; k++) {
+    CollSlot& m = c.slot(seq + (uint64_t)k);
+    if (m.seq.load(std::memory_order_acquire) != seq + (uint64_t)k || m.state.load(std::memory_order_acquire) != kSlotCollected) return true;
   }
   return false;
 }
@@ -487,7 +509,126 @@ bool ProxyEngine::plan_member(Communicator& c, CollSlot& head, CollSlot& m, cons
   return true;
 }
 
+// Ranks that share a GPU. Between two short launches of a stream the memory idles for about 4 us
+// (the last CTAs' stores, the completion word, the next kernel's first loads: two ranks x 8 MiB fp32
+// took 9.4 us a launch, 5.1 of them at the copy rate), so collectives that wait already go out
+// together (16 such calls on each of two communicators: 300 -> 199 us). Members run side by side: no byte of one may be another's (sources shared between
+// members would be safe, but are not worth a second kind of check), and all ranks' callers are on
+// the head's streams. Requests ordered by semaphores stay alone: outside a group the caller's
+// stream reaches a request's "submitted" value only behind the one before it, so a launch that
+// waited for both would wait for itself. (Other callers wait on the host until their requests have
+// been launched, at the end of the group at the latest, so what queues here is one group's.) Beyond kBatchTraffic bytes moved the gap is under a tenth of the launch.
+namespace {
+constexpr uint64_t kBatchTraffic = 256ull << 20;
+struct Span { uint64_t lo, hi; };
+// Everything a collective reads or writes, as sorted ranges that do not touch.
+int touched_by(const CollSlot& s, int nranks, Span* out) {
+  const CollOp& o0 = s.ops[0];
+  const uint64_t esz = kind_reduces(o0.kind) ? (uint64_t)dtype_size(o0.dtype) : 1;
+  const uint64_t in = send_units(o0.kind, o0.count, nranks) * esz, res = recv_units(o0.kind, o0.count, nranks) * esz;
+  Span all[2 * kMaxRanks];
+  int n = 0;
+  for (int r = 0; r < nranks; r++) {
+    all[n++] = {s.ops[r].send_va, s.ops[r].send_va + in};
+    all[n++] = {s.ops[r].recv_va, s.ops[r].recv_va + res};
+  }
+  std::sort(all, all + n, [](const Span& a, const Span& b) { return a.lo < b.lo; });
+  int m = 0;
+  for (int i = 0; i < n; i++) {
+    if (m > 0 && all[i].lo <= out[m - 1].hi) out[m - 1].hi = std::max(out[m - 1].hi, all[i].hi);
+    else out[m++] = all[i];
+  }
+  return m;
+}
+uint64_t traffic(const CollSlot& s, int nranks) {
+  const CollOp& o0 = s.ops[0];
+  const uint64_t esz = kind_reduces(o0.kind) ? (uint64_t)dtype_size(o0.dtype) : 1;
+  return (uint64_t)nranks * (send_units(o0.kind, o0.count, nranks) + recv_units(o0.kind, o0.count, nranks)) * esz;
+}
+}  // namespace
+
+void ProxyEngine::extend_one_gpu(Communicator& c, CollSlot& head, uint64_t seq, const PlanInput& head_in, uint64_t now) {
+  const CollOp& h0 = head.ops[0];
+  if (c.client_launch || head.nslices != 1 || head.plan.bounded || c.slot(seq + 1).state.load(std::memory_order_acquire) != kSlotCollected) return;
+  if (head_in.requested_variant > 0 && head_in.requested_variant != kOneGpu) return;
+  for (int r = 0; r < c.nranks; r++)
+    if (head.ops[r].sync_slot) return;
+  if (!daemon_->backend()->batch_supported(kOneGpu, head_in.dtype, head_in.op)) return;
+  const bool reduces = kind_reduces(h0.kind);
+  const uint64_t slice_bytes = daemon_->qos().slice_bytes(c.id, now);
+  Span spans[2 * kMaxRanks * kMaxBatch];
+  int nspans = touched_by(head, c.nranks, spans);
+  uint64_t bytes = head.plan.bytes, moved = traffic(head, c.nranks);
+  int len = 1;
+  while (len < kMaxBatch && moved < kBatchTraffic) {
+    const uint64_t mseq = seq + (uint64_t)len;
+    CollSlot& m = c.slot(mseq);
+    if (m.seq.load(std::memory_order_acquire) != mseq) break;
+    int expect = kSlotCollected;
+    if (!m.state.compare_exchange_strong(expect, kSlotPlanning, std::memory_order_acq_rel)) break;
+    const CollOp& o0 = m.ops[0];
+    // Anything the ranks disagree on is left to the ordinary path, which reports it.
+    bool fits = true;
+    for (int r = 0; r < c.nranks && fits; r++) {
+      const CollOp &o = m.ops[r], &h = head.ops[r];
+      fits = o.valid && o.sync_slot == 0 && o.kind == h0.kind && o.count == o0.count && (!reduces || (o.dtype == h0.dtype && o.op == h0.op && o.scale == h0.scale)) &&
+             o.variant_req == h.variant_req && o.on_caller_stream == h.on_caller_stream && o.caller_stream == h.caller_stream;
+    }
+    Plan mp;
+    Span mine[2 * kMaxRanks];
+    int nmine = 0;
+    if (fits) {
+      PlanInput in = head_in;
+      in.count = o0.count;
+      mp = daemon_->planner().plan(in);
+      fits = mp.status == proto::kOk && mp.variant == kOneGpu && moved + traffic(m, c.nranks) <= 2 * kBatchTraffic &&
+             !(slice_bytes && bytes + mp.bytes > slice_bytes);   // a tenant with competitors stays within its slices
+    }
+    if (fits) {
+      nmine = touched_by(m, c.nranks, mine);
+      for (int i = 0, j = 0; i < nmine && j < nspans && fits;) {
+        if (mine[i].hi <= spans[j].lo) i++;
+        else if (spans[j].hi <= mine[i].lo) j++;
+        else fits = false;
+      }
+    }
+    if (!fits) {
+      m.state.store(kSlotCollected, std::memory_order_release);   // planned on its own later
+      break;
+    }
+    std::copy(mine, mine + nmine, spans + nspans);
+    std::inplace_merge(spans, spans + nspans, spans + nspans + nmine, [](const Span& a, const Span& b) { return a.lo < b.lo; });
+    nspans += nmine;
+    m.plan = mp;
+    m.status = proto::kOk;
+    m.nslices = 1;
+    m.slice_count = o0.count;
+    m.batch_len = 0;
+    m.fused_kernel = false;
+    m.batch_bytes = 0;
+    m.ticket_base = head.ticket_base;
+    m.t_ready_us = now;
+    m.admitted_slices.store(0, std::memory_order_relaxed);
+    m.group_launch.store(0, std::memory_order_relaxed);
+    bytes += mp.bytes;
+    moved += traffic(m, c.nranks);
+    c.planned.fetch_add(1);
+    m.state.store(kSlotPlanned, std::memory_order_release);
+    len++;
+  }
+  if (len == 1) return;
+  head.batch_len = len;
+  head.fused_kernel = true;
+  head.batch_bytes = bytes;
+  c.fused_launches.fetch_add(1);
+  c.fused_members.fetch_add((uint64_t)len);
+}
+
 void ProxyEngine::extend_batch(Communicator& c, CollSlot& head, uint64_t seq, const PlanInput& head_in, uint64_t now) {
+  if (head.plan.variant == kOneGpu) {
+    extend_one_gpu(c, head, seq, head_in, now);
+    return;
+  }
   const int limit = std::min(daemon_->config().fuse_allreduce, kMaxBatch);
   const bool single = daemon_->config().single_through_fused;
   if (limit <= 1 && !(single && !c.client_launch)) return;   // a lone collective through the fused kernel is a daemon-launch experiment
@@ -525,6 +666,7 @@ void ProxyEngine::extend_batch(Communicator& c, CollSlot& head, uint64_t seq, co
     m.slice_count = m.ops[0].count;
     m.batch_len = 0;
     m.batch_bytes = 0;
+    m.ticket_base = head.ticket_base;
     m.t_ready_us = now;
     m.admitted_slices.store(0, std::memory_order_relaxed);
     m.group_launch.store(0, std::memory_order_relaxed);
@@ -548,6 +690,7 @@ void ProxyEngine::fill_batch_args(Communicator& c, CollSlot& head, uint64_t seq,
   memset(&b, 0, sizeof b);
   fill_args(c, head, rank, 0, &b.base);
   b.nops = head.batch_len;
+  b.kind = head.ops[0].kind;
   for (int k = 0; k < head.batch_len; k++) {
     CollSlot& m = k == 0 ? head : c.slot(seq + (uint64_t)k);
     b.count[k] = m.ops[0].count;
@@ -861,7 +1004,7 @@ bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
       c.async_error.store(rc);
       c.state.store(kCommError);
     } else {
-      r0.inflight.push_back({b.base.seq, s.batch_bytes});
+      r0.inflight.push_back({b.base.seq, s.batch_bytes, s.plan.variant == kOneGpu ? (uint64_t)s.batch_len : 1});
       r0.last_ticket.store(b.base.seq, std::memory_order_relaxed);
     }
     r0.next_slice = 1;
@@ -1095,7 +1238,7 @@ bool ProxyEngine::advance(RankState& rs) {
     if (st == kSlotCollecting) break;
     if (st == kSlotCollected) {
       if (c.paused.load(std::memory_order_acquire)) break;
-      if (followers_still_arriving(c, s, seq)) break;
+      if (followers_still_arriving(c, s, seq) || wait_for_company(c, s, seq)) break;
       int expect = kSlotCollected;
       if (!s.state.compare_exchange_strong(expect, kSlotPlanning, std::memory_order_acq_rel)) break;
       {
@@ -1176,7 +1319,7 @@ void ProxyEngine::housekeeping(RankState& rs) {
     const uint64_t done = __atomic_load_n(&rs.status->done_seq, __ATOMIC_ACQUIRE);
     while (!rs.inflight.empty() && rs.inflight.front().ticket <= done) {
       daemon_->qos().complete(c.id, rs.inflight.front().bytes);
-      c.completed.fetch_add(1);
+      c.completed.fetch_add(rs.inflight.front().members);
       rs.inflight.pop_front();
     }
   }

@@ -613,6 +613,7 @@ class CudaBackend : public Backend {
   }
 
   bool batch_supported(int variant, int dtype, int op) const override {
+    if (variant == kOneGpu) return true;
     if (variant_is_nvls(variant) && !nvls_) return false;
     return batch_kernel_function(variant, dtype, op) != nullptr;
   }
@@ -621,7 +622,7 @@ class CudaBackend : public Backend {
   }
   int launch_batch(int dev, const BatchArgs& b, LaunchDims dims, void* stream) override {
     (void)dev;
-    cudaError_t e = mccs::launch_batch(b, dims, stream);
+    cudaError_t e = b.base.variant == kOneGpu ? launch_one_gpu_batch(b, stream) : mccs::launch_batch(b, dims, stream);
     if (e != cudaSuccess) {
       LOG_ERROR("fused launch of %d x %s failed: %s", b.nops, variant_name(b.base.variant), cudaGetErrorString(e));
       cudaGetLastError();

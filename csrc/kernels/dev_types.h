@@ -155,6 +155,7 @@ enum BatchFlags : uint32_t {
 struct BatchArgs {
   CollArgs base;
   int32_t nops;
+  int32_t kind;                              // CollKind of the members: any for kOneGpu, AllReduce for the others
   uint32_t flags;                            // BatchFlags
   // Optional completion word for the caller: the last CTA of this rank to finish stores
   // `done_value` to `done_ptr` (null = nobody is told from inside the kernel).
@@ -190,6 +191,20 @@ struct OneGpuArgs {
   uint32_t* counter;         // finished CTAs, wraps to zero at the grid size; null = no completion word
   uint64_t seq;
   StatusBlock* status[kMaxRanks];
+};
+
+// Several collectives of such a communicator in one launch: same kind, type and operator, buffers
+// that share no byte. Member k has the CTAs [first[k], first[k + 1]) of grid.x, at least one; the
+// entries behind the last member are the size of the grid.
+struct OneGpuMember {
+  const void* send[kMaxRanks];
+  void* recv[kMaxRanks];
+  uint64_t count;
+};
+struct OneGpuBatchArgs {
+  OneGpuArgs base;           // what is per launch; its own send, recv and count are unused
+  uint32_t first[kMaxBatch + 1];
+  OneGpuMember member[kMaxBatch];
 };
 
 struct LaunchDims {

@@ -21,7 +21,9 @@ int max_cooperative_ctas(int variant, int dtype, int op, int threads, int nranks
 // the message.
 cudaError_t launch_one_gpu(int kind, const CollArgs& args, int max_ctas, bool completion, void* stream);
 // The kernel such a launch runs; null when there is none for this type and operator.
-const void* one_gpu_function(int kind, int dtype, int op, int nranks, bool ragged);
+const void* one_gpu_function(int kind, int dtype, int op, int nranks, bool ragged, bool batch = false);
+// Several such collectives in one launch, with a completion word (b.base.seq).
+cudaError_t launch_one_gpu_batch(const BatchArgs& b, void* stream);
 
 // Fused AllReduce (several members in one launch, see batch.cuh). Only the two-shot
 // variants have a fused form; returns null / cudaErrorInvalidDeviceFunction otherwise.

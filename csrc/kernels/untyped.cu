@@ -20,10 +20,14 @@ extern "C" const void* mccs_kfn_untyped(int variant) {
 
 extern "C" const void* mccs_kfn_local_copy_ragged() { return (const void*)&local_copy_ragged_kernel; }
 
-extern "C" const void* mccs_kfn_group_gather(int nranks, int ragged) {
-  if (nranks <= 2) return ragged ? (const void*)&group_gather_ragged_kernel<2> : (const void*)&group_gather_kernel<2>;
-  if (nranks <= 4) return ragged ? (const void*)&group_gather_ragged_kernel<4> : (const void*)&group_gather_kernel<4>;
-  return ragged ? (const void*)&group_gather_ragged_kernel<8> : (const void*)&group_gather_kernel<8>;
+template <typename Args>
+static const void* gather_by_ranks(int nranks, bool ragged) {
+  if (nranks <= 2) return ragged ? (const void*)&group_gather_ragged_kernel<2, Args> : (const void*)&group_gather_kernel<2, Args>;
+  if (nranks <= 4) return ragged ? (const void*)&group_gather_ragged_kernel<4, Args> : (const void*)&group_gather_kernel<4, Args>;
+  return ragged ? (const void*)&group_gather_ragged_kernel<8, Args> : (const void*)&group_gather_kernel<8, Args>;
+}
+extern "C" const void* mccs_kfn_group_gather(int nranks, int ragged, int batch) {
+  return batch ? gather_by_ranks<OneGpuBatchArgs>(nranks, ragged != 0) : gather_by_ranks<OneGpuArgs>(nranks, ragged != 0);
 }
 
 }  // namespace dev

@@ -1805,6 +1805,9 @@ mccsResult_t mccsGroupEnd(void) {
   mccsResult_t result = g_deferred.empty() ? mccsSuccess : flush_deferred();
   std::vector<GroupItem> items;
   items.swap(g_group_items);
+  // No more requests of this group: the daemon need not wait for company for what it holds.
+  for (const GroupItem& it : items)
+    if (it.comm->dp_status) __atomic_store_n(&it.comm->dp_status->group_closed, it.comm->next_user_seq - 1, __ATOMIC_RELEASE);
   // Collect every completion, then order each (communicator, stream) pair once.
   for (const GroupItem& it : items) {
     proto::WorkCompletion wc;

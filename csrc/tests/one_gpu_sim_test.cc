@@ -1,12 +1,14 @@
 // The one-GPU kernels of kernels/one_gpu.cuh (the source the GPU build compiles) on the SIMT
 // emulator, against plain loops: every rank count and register class, counts around the pack
-// and tile edges, every combination of 16-byte phases, in place, bounded grids. Guard bytes
+// and tile edges, every combination of 16-byte phases, in place, bounded grids, several
+// collectives in one launch. Guard bytes
 // around every output catch a store outside it, the emulator a misaligned access.
 #include "sim/simt_sim.h"
 
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <random>
 #include <type_traits>
 
@@ -42,8 +44,8 @@ template <typename T> T made(double v) { return (T)v; }
 template <> __nv_bfloat16 made(double v) { return __float2bfloat16_rn((float)v); }
 template <> __half made(double v) { return __float2half_rn((float)v); }
 
-template <typename Kernel>
-void launch(Kernel k, const OneGpuArgs& a, int ctas, int groups, int threads) {
+template <typename Kernel, typename Args>
+void launch(Kernel k, const Args& a, int ctas, int groups, int threads) {
   std::vector<std::thread> pool;
   sim::Dim3 grid;
   grid.x = (unsigned)ctas;
@@ -174,6 +176,75 @@ void copy_case(size_t count, size_t send_off, size_t recv_off, int ctas, int thr
   free(pad);
 }
 
+// Several collectives in one launch: each member against plain loops, whatever CTAs it has (first[]
+// as the launcher fills it, one CTA at least, `per` packs' worth of bytes each).
+void batch_case(int kind, int n, const std::vector<size_t>& counts, size_t send_off, size_t recv_off, size_t per, int threads) {
+  const bool gather = kind == kAllGather, scatter = kind == kReduceScatter;
+  const size_t esz = gather ? 1 : sizeof(float), nn = (size_t)n;
+  std::vector<Block> send, recv;
+  send.reserve(counts.size() * nn);   // (blocks must not move)
+  recv.reserve(counts.size() * nn);
+  OneGpuBatchArgs b;
+  memset(&b, 0, sizeof b);
+  uint64_t bits = 0;
+  unsigned ctas = 0;
+  for (size_t k = 0; k < (size_t)kMaxBatch; k++) {
+    b.first[k] = ctas;
+    if (k >= counts.size()) continue;
+    const size_t c = counts[k];
+    ctas += (unsigned)std::max<size_t>((c * esz + per - 1) / per, 1);
+    b.member[k].count = c;
+    bits |= kind == kAllReduce ? 0 : c * esz;
+    for (int r = 0; r < n; r++) {
+      send.emplace_back(c * esz * (scatter ? nn : 1), send_off * esz);
+      recv.emplace_back(c * esz * (gather ? nn : 1), recv_off * esz);
+      uint8_t* sp = send.back().p();
+      for (size_t i = 0; i < send.back().bytes / esz; i++) {
+        if (gather) sp[i] = (uint8_t)(i * 7 + (size_t)r * 31 + k);
+        else ((float*)sp)[i] = (float)((i * 3 + (size_t)r * 5 + k) % 23);
+      }
+      b.member[k].send[r] = sp;
+      b.member[k].recv[r] = recv.back().p();
+      bits |= (uint64_t)sp | (uint64_t)recv.back().p();
+    }
+  }
+  b.first[kMaxBatch] = ctas;
+  std::vector<StatusBlock> status(nn);
+  uint32_t counter = 0;
+  for (int r = 0; r < n; r++) { memset(&status[(size_t)r], 0, sizeof(StatusBlock)); b.base.status[r] = &status[(size_t)r]; }
+  b.base.nranks = n; b.base.kind = kind; b.base.op = kSum; b.base.scale = 1.0f; b.base.counter = &counter; b.base.seq = 9;
+  const bool ragged = (bits & 15u) != 0;
+  const int groups = kind == kAllReduce ? 1 : n;
+  auto go = [&](auto plain, auto rag) { ragged ? launch(rag, b, (int)ctas, groups, threads) : launch(plain, b, (int)ctas, groups, threads); };
+  using B = OneGpuBatchArgs;
+  if (gather) {
+    if (n <= 2) go(group_gather_kernel<2, B>, group_gather_ragged_kernel<2, B>);
+    else if (n <= 4) go(group_gather_kernel<4, B>, group_gather_ragged_kernel<4, B>);
+    else go(group_gather_kernel<8, B>, group_gather_ragged_kernel<8, B>);
+  } else {
+    if (n <= 2) go(group_reduce_kernel<float, OpSum, 2, B>, group_reduce_ragged_kernel<float, OpSum, 2, B>);
+    else if (n <= 4) go(group_reduce_kernel<float, OpSum, 4, B>, group_reduce_ragged_kernel<float, OpSum, 4, B>);
+    else go(group_reduce_kernel<float, OpSum, 8, B>, group_reduce_ragged_kernel<float, OpSum, 8, B>);
+  }
+  bool good = counter == 0;
+  for (size_t k = 0; k < counts.size(); k++)
+    for (size_t r = 0; r < nn; r++) {
+      Block& out = recv[k * nn + r];
+      for (size_t i = 0; i < out.bytes / esz; i++) {
+        if (gather) {
+          good &= out.p()[i] == send[k * nn + i / counts[k]].p()[i % counts[k]];
+        } else {
+          float want = 0;
+          for (size_t q = 0; q < nn; q++) want += ((const float*)send[k * nn + q].p())[(scatter ? r * counts[k] : 0) + i];
+          good &= ((const float*)out.p())[i] == want;
+        }
+      }
+      good &= out.guards_intact() && status[r].done_seq == 9;
+    }
+  g_cases++;
+  if (!good) { g_failed++; fprintf(stderr, "FAILED: batch kind %d n %d members %zu ragged %d per %zu\n", kind, n, counts.size(), ragged, per); }
+}
+
 template <typename T>
 void type_cases() {
   const size_t per = 16 / sizeof(T);
@@ -216,6 +287,14 @@ int main() {
       gather_case(n, count, mixed, same, false, 2, 64);
       gather_case(n, count, zero, mixed, true, 2, 32);
     }
+  for (int kind : {(int)kAllReduce, (int)kAllGather, (int)kReduceScatter})
+    for (int n : {2, 3, 4, 8})
+      for (size_t per : {(size_t)512, (size_t)1024}) {   // the tile of 32 threads is 512 bytes (one pack each) or a multiple
+        batch_case(kind, n, {64, 1024, 16, 512}, 0, 0, per, 32);
+        batch_case(kind, n, {1, 130, 4099, 7, 1000, 33, 2048, 1}, 0, 0, per, 32);
+        batch_case(kind, n, {515, 515}, 3, 1, per, 32);
+        batch_case(kind, n, {48}, 0, 0, per, 32);
+      }
   for (size_t count : {(size_t)1, (size_t)15, (size_t)16, (size_t)31, (size_t)2048, (size_t)2049, (size_t)5003})
     for (size_t so = 0; so < 16; so++)
       for (size_t ro : {(size_t)0, (size_t)1, (size_t)8, (size_t)15}) copy_case(count, so, ro, 2, 32);

@@ -62,7 +62,7 @@ def render(stats: dict) -> str:
     comms = stats.get("communicators", {})
     per_comm = [
         ("mccs_comm_planned_total", "counter", "collectives planned", "planned"),
-        ("mccs_comm_completed_total", "counter", "kernel launches completed (a fused launch counts once)", "completed"),
+        ("mccs_comm_completed_total", "counter", "kernel launches completed (a launch fused by fuse_allreduce counts once)", "completed"),
         ("mccs_comm_fused_launches_total", "counter", "launches that carried several AllReduces", "fused_launches"),
         ("mccs_comm_fused_members_total", "counter", "AllReduces carried by fused launches", "fused_members"),
         ("mccs_comm_config_epoch", "gauge", "live reconfigurations applied", "config_epoch"),

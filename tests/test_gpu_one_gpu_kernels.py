@@ -4,6 +4,9 @@ and a grid of many tiles, buffers at other 16-byte phases, in place, and a grid 
 operator's CTA limit. Sums accumulate in fp32 (fp64 for doubles) in rank order and are rounded
 once, so the result differs from the fp64 sum by at most n - 1 roundings of partial sums below n
 in magnitude plus the final rounding."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -99,3 +102,65 @@ def test_one_gpu_sizes_and_phases(service, coll, n):
 def test_one_gpu_integer_types(service, dtype):
     _case(service, "all_reduce", 4, dtype, 10_007, op="max")
     _case(service, "reduce_scatter", 8, dtype, 4_099, op="max")
+
+
+@pytest.mark.parametrize("coll,n", [("all_reduce", 2), ("all_reduce", 8), ("reduce_scatter", 4), ("all_gather", 3)])
+def test_one_gpu_groups_in_one_launch(service, coll, n):
+    """Collectives of one group may share a launch: different lengths (below a pack, around a tile,
+    ragged), and calls that have to run in order: a chain in place, and one that reads what the
+    chain left with other ranks. In odd rounds the communicator is paused until the whole group
+    waits, in even ones products queued in front keep the GPU busy while it is posted."""
+    M = service
+    torch.cuda.set_device(0)
+    counts = [4096, 1, 300_008, 65_536, 8, 77, 4096, 1 << 20, 4096, 4096]
+    cid, comms = fresh_comm_id(), [None] * n
+    run_ranks(n, lambda r: comms.__setitem__(r, M.Communicator(cid, r, n, device=0)))
+    keep = []
+
+    def per_rank(count):
+        bufs = [M.Buffer(count * 4, 0) for _ in range(n)]
+        keep.extend(bufs)
+        return [b.tensor(torch.float32, count) for b in bufs]
+
+    pairs = [(per_rank(c * (n if coll == "reduce_scatter" else 1)), per_rank(c * (n if coll == "all_gather" else 1))) for c in counts]
+    chain, last = per_rank(50_000), per_rank(50_000)
+    big = torch.randn(4096, 4096, device="cuda")
+    for it in range(4):
+        for k, (send, _) in enumerate(pairs):
+            for r in range(n):
+                send[r].copy_(torch.arange(send[r].numel(), device="cuda") % 13 + r + k + it)   # sums of small whole numbers are exact
+        for r in range(n):
+            chain[r].fill_(1.0)
+        if it % 2:
+            assert M.daemon.embedded_admin({"cmd": "pause", "communicator_id": cid})["status"] == "ok"
+            threading.Timer(0.1, lambda: M.daemon.embedded_admin({"cmd": "resume", "communicator_id": cid})).start()
+        else:
+            for _ in range(6):
+                torch.mm(big, big)
+        with M.group():
+            for send, recv in pairs:
+                for r in range(n):
+                    getattr(comms[r], coll)(send[r], recv[r])
+            for _ in range(3):
+                for r in range(n):
+                    comms[r].all_reduce(chain[r])
+            for r in range(n):
+                comms[r].all_reduce(chain[(r + 1) % n], last[r])
+        for k, (send, recv) in enumerate(pairs):
+            count = counts[k]
+            whole = torch.cat(send) if coll == "all_gather" else torch.stack(send).sum(0)
+            for r in range(n):
+                want = whole[r * count:(r + 1) * count] if coll == "reduce_scatter" else whole
+                assert torch.equal(recv[r], want), f"{coll} n={n} member {k} ({count})"
+        for r in range(n):
+            assert bool((chain[r] == float(n) ** 3).all()) and bool((last[r] == float(n) ** 4).all())
+    for _ in range(200):         # the daemon counts a launch's members once it has seen the completion word
+        q = comms[0].query()
+        if q["launched"] == q["completed"]:
+            break
+        time.sleep(0.01)
+    assert q["async_error"] == 0 and q["device_error"] == 0 and q["launched"] == q["completed"] == 4 * (len(counts) + 4)
+    stats = M.daemon.embedded_admin({"cmd": "stats"})["stats"]["communicators"][str(cid)]
+    assert stats["fused_members"] >= 2 * len(counts)      # both paused rounds: every independent call shared a launch
+    for c in comms:
+        c.destroy()
