@@ -551,6 +551,9 @@ void ProxyEngine::extend_one_gpu(Communicator& c, CollSlot& head, uint64_t seq, 
   const CollOp& h0 = head.ops[0];
   if (c.client_launch || head.nslices != 1 || head.plan.bounded || c.slot(seq + 1).state.load(std::memory_order_acquire) != kSlotCollected) return;
   if (head_in.requested_variant > 0 && head_in.requested_variant != kOneGpu) return;
+  // A window schedule admits collective by collective: one that is let in just before its window
+  // ends must not bring seven more along, and `enforce_step` counts each of them as a round.
+  if (daemon_->qos().scheduled(c.id)) return;
   for (int r = 0; r < c.nranks; r++)
     if (head.ops[r].sync_slot) return;
   if (!daemon_->backend()->batch_supported(kOneGpu, head_in.dtype, head_in.op)) return;

@@ -108,6 +108,11 @@ uint64_t QosArbiter::slice_bytes(uint32_t id, uint64_t now_us) {
   return 0;
 }
 
+bool QosArbiter::scheduled(uint32_t id) {
+  std::lock_guard<std::mutex> g(mu_);
+  return schedule_.count(id) != 0;
+}
+
 int QosArbiter::stream_priority(uint32_t id) {
   std::lock_guard<std::mutex> g(mu_);
   return tenant(id).cfg.priority > 0 ? 1 : 0;

@@ -59,6 +59,8 @@ class QosArbiter {
   int cta_cap(uint32_t id, uint64_t now_us, uint64_t stream = 0);
   // Bytes per time slice for a collective planned now (0 = do not slice).
   uint64_t slice_bytes(uint32_t id, uint64_t now_us);
+  // Whether a window schedule applies to this tenant (its windows and rounds count launches).
+  bool scheduled(uint32_t id);
   int stream_priority(uint32_t id);   // 0 normal, 1 high
 
   // A planned collective (or slice) asks to launch. `wall_us` is the Unix clock used

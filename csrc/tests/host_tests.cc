@@ -443,6 +443,7 @@ static void test_qos() {
   std::map<uint32_t, QosIntervalConfig> sched;
   sched[1].intervals = {{0, 1000}};
   r.set_schedule(10000, sched);
+  CHECK(r.scheduled(sched.begin()->first) && !r.scheduled(12345));
   r.complete(1, 64u << 20);
   // Tenant 2 was waiting all along and is behind in virtual time: it goes first.
   CHECK(r.admit(1, 1024, 12, 500) == kQosDeferFairness);
