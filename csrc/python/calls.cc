@@ -273,7 +273,8 @@ PyObject* all_gather(PyObject* self_, PyObject* const* args, Py_ssize_t nargs, P
 
 // self_copy(send, recv, stream) -> bool. Any collective of a communicator of one rank whose tensors
 // are plain memory of its GPU: one copy kernel on them where they are. False when that does not apply
-// (more ranks, other devices, other layouts, differing types) and the caller has to stage.
+// (more ranks, other devices, other layouts, differing types, ranges that overlap in part) and the caller
+// has to stage.
 PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   Calls* self = (Calls*)self_;
   if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "self_copy(send, recv, stream)"); return nullptr; }
@@ -282,11 +283,12 @@ PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   if (!out || !in->is_cuda() || !out->is_cuda() || in->get_device() != self->device || out->get_device() != self->device ||
       in->scalar_type() != out->scalar_type() || in->numel() != out->numel() || in->numel() == 0 || !in->is_contiguous() || !out->is_contiguous())
     Py_RETURN_FALSE;
-  uint64_t stream;
-  if (!resolve_stream(self, args[2], &stream)) return nullptr;
   const void* const from = in->data_ptr();
   void* const to = out->data_ptr();
   const size_t bytes = (size_t)in->numel() * (size_t)in->element_size();
+  if (from != to && (from < to ? (const char*)to - (const char*)from : (const char*)from - (const char*)to) < (ptrdiff_t)bytes) Py_RETURN_FALSE;
+  uint64_t stream;
+  if (!resolve_stream(self, args[2], &stream)) return nullptr;
   mccsResult_t rc;
   const mccsComm_t comm = self->comm;
   Py_BEGIN_ALLOW_THREADS

@@ -1741,6 +1741,9 @@ mccsResult_t mccsCommSelfCopy(mccsComm_t comm, const void* send, void* recv, siz
   if (!mccsCommTakesAnyMemory(comm) || (comm->caller_streams && (comm->deferred_wait || stream == (mccsStream_t)CU_STREAM_PER_THREAD)))
     return mccsUnsupported;
   if (bytes > (1ull << 44) || !send || !recv) return mccsInvalidArgument;
+  // The kernel reads and writes in parallel: a range that overlaps the other in part has no order.
+  const uint64_t from = (uint64_t)send, to = (uint64_t)recv;
+  if (from != to && (from < to ? to - from : from - to) < bytes) return mccsInvalidArgument;
   proto::WorkRequest wr;
   memset(&wr, 0, sizeof wr);
   wr.kind = kAllGather;

@@ -73,6 +73,10 @@ def shim() -> ctypes.CDLL:
     lib.mccsReduceScatterEx.restype = c_int
     lib.mccsAllGatherEx.argtypes = [c_void_p, c_void_p, c_void_p, c_size_t, c_int, c_void_p]
     lib.mccsAllGatherEx.restype = c_int
+    lib.mccsCommTakesAnyMemory.argtypes = [c_void_p]
+    lib.mccsCommTakesAnyMemory.restype = c_int
+    lib.mccsCommSelfCopy.argtypes = [c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]
+    lib.mccsCommSelfCopy.restype = c_int
     lib.mccsGroupStart.restype = c_int
     lib.mccsGroupEnd.restype = c_int
     lib.mccsCommQuery.argtypes = [c_void_p, POINTER(CommInfo)]
