@@ -150,7 +150,9 @@ mccsResult_t mccsReduceScatterEx(mccsComm_t comm, const void* send, void* recv, 
  * (nothing when they are equal). Unlike the collective calls this takes any memory of the
  * communicator's GPU, because no other process ever addresses it; it is planned, admitted and counted
  * like them. mccsCommTakesAnyMemory tells whether a communicator can (1) or not (0: more ranks, no
- * GPU, or a daemon in another process that launches the kernels), mccsUnsupported otherwise.
+ * GPU, or a daemon in another process that launches the kernels), mccsUnsupported otherwise; the call
+ * gives mccsUnsupported as well where its kernel would be launched after the call returns (inside a
+ * group, with a deferred wait).
  * Buffers that overlap without being the same range are refused (mccsInvalidArgument). */
 int mccsCommTakesAnyMemory(mccsComm_t comm);
 mccsResult_t mccsCommSelfCopy(mccsComm_t comm, const void* send, void* recv, size_t bytes, mccsStream_t stream);

@@ -1740,6 +1740,10 @@ int mccsCommTakesAnyMemory(mccsComm_t comm) {
 mccsResult_t mccsCommSelfCopy(mccsComm_t comm, const void* send, void* recv, size_t bytes, mccsStream_t stream) {
   if (!mccsCommTakesAnyMemory(comm) || (comm->caller_streams && (comm->deferred_wait || stream == (mccsStream_t)CU_STREAM_PER_THREAD)))
     return mccsUnsupported;
+  // Inside a group a request may only be posted: its kernel would read the buffer after whatever the
+  // caller queues next, when that memory may have been handed out again. (Nothing holds it, unlike
+  // memory of the service.)
+  if (g_group_depth > 0 && (comm->caller_streams || comm->group_defer)) return mccsUnsupported;
   if (bytes > (1ull << 44) || !send || !recv) return mccsInvalidArgument;
   // The kernel reads and writes in parallel: a range that overlaps the other in part has no order.
   const uint64_t from = (uint64_t)send, to = (uint64_t)recv;

@@ -1,10 +1,14 @@
 """The functions of ``mccs_b200.ops`` on a communicator of one rank and ordinary CUDA tensors: one copy
 kernel from tensor to tensor where that is the same as the staged form (copy into the communicator's
 arena, collective there, copy out), the staged form everywhere else."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
-from helpers import fresh_comm_id
+from helpers import REPO, fresh_comm_id
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +55,52 @@ def test_the_c_call_refuses_partial_overlap(comm):
     assert call(0, 100, 100) == 0 and call(0, 0, 100) == 0
     torch.cuda.synchronize()
     assert torch.equal(x[100:200], x[:100]) and int(x[200]) == 200
+
+
+GROUP = r"""
+import os, sys, threading
+import torch
+import mccs_b200 as M
+from mccs_b200 import ops
+
+def check(comm, pause):
+    # In each pass the input is a temporary whose block the allocator hands out again at once, and the
+    # output is read within the group: both are right only if the input was read during the call.
+    for fn in (ops.all_reduce, ops.all_gather, ops.reduce_scatter):
+        for it in range(8):
+            a = torch.full((1 << 20,), float(it + 1), device="cuda")
+            out = torch.zeros(1 << 20, device="cuda")
+            if pause and it == 0:
+                pause()
+            with M.group():
+                t = a * 2
+                at = t.data_ptr()
+                fn(comm, t, out)
+                del t
+                b = torch.full((1 << 20,), -1.0, device="cuda")
+                reused = b.data_ptr() == at
+                seen = out.clone()
+            torch.cuda.synchronize()
+            assert bool((out == 2.0 * (it + 1)).all()) and bool((seen == out).all()), (fn.__name__, it, reused)
+
+torch.cuda.set_device(0)
+mode = sys.argv[1]
+M.init(M.daemon.start_embedded(prefix=f"/tmp/mccs-group-{os.getpid()}", listen_port=-1,
+                               extra='launch = "client"\nfuse_allreduce = 4' if mode == "client" else ""))
+comm = M.Communicator(31, 0, 1, device=0)
+assert comm.launch_mode == mode
+def pause():       # the communicator answers nothing for a while
+    assert M.daemon.embedded_admin({"cmd": "pause", "communicator_id": 31})["status"] == "ok"
+    threading.Timer(0.2, lambda: M.daemon.embedded_admin({"cmd": "resume", "communicator_id": 31})).start()
+check(comm, pause)
+comm.destroy()
+M.finalize()
+M.daemon.stop_embedded()
+print("OK")
+"""
+
+
+@pytest.mark.parametrize("mode", ["daemon", "client"])
+def test_inside_a_group_the_input_is_read_during_the_call(mode):
+    p = subprocess.run([sys.executable, "-c", GROUP, mode], env=dict(os.environ, PYTHONPATH=REPO), capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and p.stdout.strip().endswith("OK"), p.stdout[-2000:] + p.stderr[-3000:]
