@@ -13,6 +13,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda.h>
 #include <dlfcn.h>
@@ -271,17 +272,24 @@ PyObject* all_gather(PyObject* self_, PyObject* const* args, Py_ssize_t nargs, P
   Py_RETURN_NONE;
 }
 
+// Whether the bytes behind a tensor are its values: no conjugation, sign or zero that torch applies
+// when it reads them, no wrapper or mode that has to see the operation.
+bool plain_bytes(const at::Tensor& t) {
+  return !t.is_conj() && !t.is_neg() && !t._is_zerotensor() && !t.is_quantized() && !at::isTensorSubclassLike(t);
+}
+
 // self_copy(send, recv, stream) -> bool. Any collective of a communicator of one rank whose tensors
 // are plain memory of its GPU: one copy kernel on them where they are. False when that does not apply
-// (more ranks, other devices, other layouts, differing types, ranges that overlap in part) and the caller
-// has to stage.
+// (more ranks, other devices, other layouts, differing types, values that are not the bytes, ranges that
+// overlap in part) and the caller has to stage.
 PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   Calls* self = (Calls*)self_;
   if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "self_copy(send, recv, stream)"); return nullptr; }
   const at::Tensor* in = self->any_memory ? tensor(args[0]) : nullptr;
   const at::Tensor* out = in ? tensor(args[1]) : nullptr;
   if (!out || !in->is_cuda() || !out->is_cuda() || in->get_device() != self->device || out->get_device() != self->device ||
-      in->scalar_type() != out->scalar_type() || in->numel() != out->numel() || in->numel() == 0 || !in->is_contiguous() || !out->is_contiguous())
+      in->scalar_type() != out->scalar_type() || in->numel() != out->numel() || in->numel() == 0 || !plain_bytes(*in) || !plain_bytes(*out) ||
+      !in->is_contiguous() || !out->is_contiguous())
     Py_RETURN_FALSE;
   const void* const from = in->data_ptr();
   void* const to = out->data_ptr();

@@ -104,3 +104,25 @@ print("OK")
 def test_inside_a_group_the_input_is_read_during_the_call(mode):
     p = subprocess.run([sys.executable, "-c", GROUP, mode], env=dict(os.environ, PYTHONPATH=REPO), capture_output=True, text=True, timeout=300)
     assert p.returncode == 0 and p.stdout.strip().endswith("OK"), p.stdout[-2000:] + p.stderr[-3000:]
+
+
+def test_views_whose_bytes_are_not_their_values(comm):
+    """Negative views (lazy, contiguous) keep their sign as input and as output; a conjugate view cannot be
+    gathered as bytes and is refused."""
+    from mccs_b200 import ops
+    x = torch.arange(1000.0, device="cuda")
+    for fn in _collectives():
+        if fn.__name__ != "all_gather":        # bytes of a negative view: refused like those of a conjugate one
+            out = torch.zeros_like(x)
+            fn(comm, torch._neg_view(x), out)
+            assert torch.equal(out, -x)
+            store = torch.zeros_like(x)
+            fn(comm, x, torch._neg_view(store))
+            assert torch.equal(store, -x)
+    z = torch.randn(64, dtype=torch.complex64, device="cuda")
+    for send in (z.conj(), torch._neg_view(x)):
+        with pytest.raises(RuntimeError):
+            ops.all_gather(comm, send, torch.empty_like(send))
+    out = torch.empty_like(z)
+    ops.all_gather(comm, z, out)               # without the view it is plain memory
+    assert torch.equal(out, z)
