@@ -30,6 +30,7 @@ decltype(&mccsAllGatherEx) g_all_gather;
 decltype(&mccsReduceScatterEx) g_reduce_scatter;
 decltype(&mccsCommSelfCopy) g_self_copy;
 decltype(&mccsCommTakesAnyMemory) g_takes_any_memory;
+decltype(&mccsMemInfo) g_mem_info;
 decltype(&mccsGroupStart) g_group_start;
 decltype(&mccsGroupEnd) g_group_end;
 
@@ -56,8 +57,8 @@ struct Calls {
 
 const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
-// mccsDataType_t of a tensor; KeyError with the type, as the dictionary raises it, for another one.
-bool type_code(const at::Tensor& t, PyObject* of, int* out) {
+// mccsDataType_t of a tensor, if there is one.
+bool known_type(const at::Tensor& t, int* out) {
   switch (t.scalar_type()) {
     case at::kChar: *out = mccsInt8; return true;
     case at::kByte: *out = mccsUint8; return true;
@@ -69,8 +70,13 @@ bool type_code(const at::Tensor& t, PyObject* of, int* out) {
     case at::kFloat: *out = mccsFloat32; return true;
     case at::kDouble: *out = mccsFloat64; return true;
     case at::kBFloat16: *out = mccsBfloat16; return true;
-    default: break;
+    default: return false;
   }
+}
+
+// The same; KeyError with the type, as the dictionary raises it, when there is none.
+bool type_code(const at::Tensor& t, PyObject* of, int* out) {
+  if (known_type(t, out)) return true;
   PyObject* d = PyObject_GetAttrString(of, "dtype");
   if (d) {
     PyErr_SetObject(PyExc_KeyError, d);
@@ -297,13 +303,17 @@ PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   if (from != to && (from < to ? (const char*)to - (const char*)from : (const char*)from - (const char*)to) < (ptrdiff_t)bytes) Py_RETURN_FALSE;
   uint64_t stream;
   if (!resolve_stream(self, args[2], &stream)) return nullptr;
+  // Memory of the service is named as such: the request then keeps it from being freed while it waits.
+  int dtype;
+  const bool service = g_mem_info(from, nullptr, nullptr, nullptr) == mccsSuccess && g_mem_info(to, nullptr, nullptr, nullptr) == mccsSuccess;
+  if (service && !known_type(*in, &dtype)) Py_RETURN_FALSE;
   mccsResult_t rc;
   const mccsComm_t comm = self->comm;
   Py_BEGIN_ALLOW_THREADS
-  rc = g_self_copy(comm, from, to, bytes, (mccsStream_t)stream);
+  rc = service ? g_all_gather(comm, from, to, bytes, mccsAlgoAuto, (mccsStream_t)stream) : g_self_copy(comm, from, to, bytes, (mccsStream_t)stream);
   Py_END_ALLOW_THREADS
-  if (rc == mccsUnsupported) Py_RETURN_FALSE;
-  if (rc != mccsSuccess) return raise(rc, "mccsCommSelfCopy");
+  if (rc == mccsUnsupported && !service) Py_RETURN_FALSE;
+  if (rc != mccsSuccess) return raise(rc, service ? "mccsAllGather" : "mccsCommSelfCopy");
   Py_RETURN_TRUE;
 }
 
@@ -427,9 +437,9 @@ PyObject* local_all_reduce(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 // bind(functions, Buffer, dtypes, ops, algos, MccsError, capturing)
 PyObject* module_bind(PyObject*, PyObject* args) {
-  unsigned long long ar, ag, rs, gs, ge, sc, am;
+  unsigned long long ar, ag, rs, gs, ge, sc, am, mi;
   PyObject *buffer, *dtypes, *ops, *algos, *error, *capturing;
-  if (!PyArg_ParseTuple(args, "(KKKKKKK)OO!O!O!OO", &ar, &ag, &rs, &gs, &ge, &sc, &am, &buffer, &PyDict_Type, &dtypes, &PyDict_Type, &ops,
+  if (!PyArg_ParseTuple(args, "(KKKKKKKK)OO!O!O!OO", &ar, &ag, &rs, &gs, &ge, &sc, &am, &mi, &buffer, &PyDict_Type, &dtypes, &PyDict_Type, &ops,
                         &PyDict_Type, &algos, &error, &capturing))
     return nullptr;
   g_all_reduce = (decltype(g_all_reduce))ar;
@@ -439,6 +449,7 @@ PyObject* module_bind(PyObject*, PyObject* args) {
   g_group_end = (decltype(g_group_end))ge;
   g_self_copy = (decltype(g_self_copy))sc;
   g_takes_any_memory = (decltype(g_takes_any_memory))am;
+  g_mem_info = (decltype(g_mem_info))mi;
   g_buffer_type = Py_NewRef(buffer);
   g_dtypes = Py_NewRef(dtypes);
   g_ops = Py_NewRef(ops);

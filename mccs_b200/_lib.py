@@ -121,6 +121,18 @@ def daemon_lib() -> ctypes.CDLL:
     return lib
 
 
+def bind_calls(mod, **stand_ins) -> None:
+    """Gives the extension the shim's functions, or a test's stand-ins for some of them."""
+    import torch
+
+    from . import client
+    lib = shim()
+    mod.bind(tuple(ctypes.cast(stand_ins.get(f) or getattr(lib, f), c_void_p).value for f in
+                   ("mccsAllReduceEx", "mccsAllGatherEx", "mccsReduceScatterEx", "mccsGroupStart", "mccsGroupEnd", "mccsCommSelfCopy",
+                    "mccsCommTakesAnyMemory", "mccsMemInfo")),
+             client.Buffer, client.DTYPES, client.OPS, client.ALGOS, MccsError, torch.cuda.is_current_stream_capturing)
+
+
 _calls = None
 _calls_lock = threading.Lock()
 
@@ -137,21 +149,14 @@ def calls():
         import importlib.machinery
         import importlib.util
 
-        import torch
-
-        from . import client
+        import torch  # noqa: F401  (the extension links against its libraries)
         path = os.path.join(NATIVE_DIR, "_calls.so")
         if not os.path.exists(path):
             raise ImportError(f"{path} is missing: build the native code with `make -j` at the repository root")
         loader = importlib.machinery.ExtensionFileLoader("mccs_b200._calls", path)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("mccs_b200._calls", loader))
         loader.exec_module(mod)
-        lib = shim()
-        mod.bind(tuple(ctypes.cast(getattr(lib, f), c_void_p).value for f in
-                       ("mccsAllReduceEx", "mccsAllGatherEx", "mccsReduceScatterEx", "mccsGroupStart", "mccsGroupEnd", "mccsCommSelfCopy",
-                        "mccsCommTakesAnyMemory")),
-                 client.Buffer, client.DTYPES, client.OPS, client.ALGOS, MccsError,
-                 torch.cuda.is_current_stream_capturing)
+        bind_calls(mod)
         _calls = mod
     return _calls
 

@@ -1,6 +1,7 @@
 """The functions of ``mccs_b200.ops`` on a communicator of one rank and ordinary CUDA tensors: one copy
 kernel from tensor to tensor where that is the same as the staged form (copy into the communicator's
 arena, collective there, copy out), the staged form everywhere else."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -126,3 +127,30 @@ def test_views_whose_bytes_are_not_their_values(comm):
     out = torch.empty_like(z)
     ops.all_gather(comm, z, out)               # without the view it is plain memory
     assert torch.equal(out, z)
+
+
+def test_service_memory_is_named_to_the_daemon(service):
+    """Two tensors in service memory go out as an ordinary collective, whose request keeps the allocations from
+    being released while it waits; with a tensor of the caller's own it is the direct copy. (Seen at
+    stand-ins for the C functions: nothing is launched.)"""
+    from mccs_b200 import _lib
+    mod, called = _lib.calls(), []
+    gather = ctypes.CFUNCTYPE(ctypes.c_int, *[ctypes.c_void_p] * 3, ctypes.c_size_t, ctypes.c_int, ctypes.c_void_p)(
+        lambda c, s, d, n, algo, st: called.append(("gather", s, d, n)) or 0)
+    copy = ctypes.CFUNCTYPE(ctypes.c_int, *[ctypes.c_void_p] * 3, ctypes.c_size_t, ctypes.c_void_p)(
+        lambda c, s, d, n, st: called.append(("copy", s, d, n)) or 0)
+    any_memory = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p)(lambda c: 1)
+    torch.cuda.set_device(0)
+    bufs = [service.Buffer(4096, 0) for _ in range(2)]
+    a, b = (x.tensor(torch.float32) for x in bufs)
+    short, x = bufs[1].tensor(torch.int16), torch.zeros(1024, device="cuda")
+    try:
+        _lib.bind_calls(mod, mccsAllGatherEx=gather, mccsCommSelfCopy=copy, mccsCommTakesAnyMemory=any_memory)
+        calls = mod.CommCalls()
+        calls._attach(1, 0, 1)
+        assert calls.self_copy(a, b, None) is True and called.pop() == ("gather", a.data_ptr(), b.data_ptr(), 4096)
+        assert calls.self_copy(a, x, None) is True and called.pop() == ("copy", a.data_ptr(), x.data_ptr(), 4096)
+        assert calls.self_copy(x, b, None) is True and called.pop() == ("copy", x.data_ptr(), b.data_ptr(), 4096)
+        assert calls.self_copy(bufs[0].tensor(torch.int16), short, None) is False and not called    # no collective of this type
+    finally:
+        _lib.bind_calls(mod)
