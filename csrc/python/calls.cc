@@ -14,11 +14,14 @@
 #include <Python.h>
 
 #include <ATen/TensorSubclassLikeUtils.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/InferenceMode.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda.h>
 #include <dlfcn.h>
 #include <stdint.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/variable.h>
 
 #include "../include/mccs.h"
 #include "../include/mccs_noalloc.h"
@@ -284,6 +287,13 @@ bool plain_bytes(const at::Tensor& t) {
   return !t.is_conj() && !t.is_neg() && !t._is_zerotensor() && !t.is_quantized() && !at::isTensorSubclassLike(t);
 }
 
+// Whether writing `out` from `in` concerns autograd beyond the version of `out`: what copy_ records, or
+// refuses, is left to copy_.
+bool autograd_takes_part(const at::Tensor& in, const at::Tensor& out) {
+  return (at::GradMode::is_enabled() && (in.requires_grad() || out.requires_grad())) || in._fw_grad(0).defined() || out._fw_grad(0).defined() ||
+         (out.is_inference() && !c10::InferenceMode::is_enabled());
+}
+
 // self_copy(send, recv, stream) -> bool. Any collective of a communicator of one rank whose tensors
 // are plain memory of its GPU: one copy kernel on them where they are. False when that does not apply
 // (more ranks, other devices, other layouts, differing types, values that are not the bytes, ranges that
@@ -306,13 +316,14 @@ PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   // Memory of the service is named as such: the request then keeps it from being freed while it waits.
   int dtype;
   const bool service = g_mem_info(from, nullptr, nullptr, nullptr) == mccsSuccess && g_mem_info(to, nullptr, nullptr, nullptr) == mccsSuccess;
-  if (service && !known_type(*in, &dtype)) Py_RETURN_FALSE;
+  if (service ? !known_type(*in, &dtype) : autograd_takes_part(*in, *out)) Py_RETURN_FALSE;
   mccsResult_t rc;
   const mccsComm_t comm = self->comm;
   Py_BEGIN_ALLOW_THREADS
   rc = service ? g_all_gather(comm, from, to, bytes, mccsAlgoAuto, (mccsStream_t)stream) : g_self_copy(comm, from, to, bytes, (mccsStream_t)stream);
   Py_END_ALLOW_THREADS
   if (rc == mccsUnsupported && !service) Py_RETURN_FALSE;
+  if (rc == mccsSuccess && !service && !out->is_inference()) torch::autograd::impl::bump_version(*out);   // as copy_ does
   if (rc != mccsSuccess) return raise(rc, service ? "mccsAllGather" : "mccsCommSelfCopy");
   Py_RETURN_TRUE;
 }

@@ -154,3 +154,38 @@ def test_service_memory_is_named_to_the_daemon(service):
         assert calls.self_copy(bufs[0].tensor(torch.int16), short, None) is False and not called    # no collective of this type
     finally:
         _lib.bind_calls(mod)
+
+
+def test_autograd_sees_the_write(comm):
+    """What ``copy_`` into the output did: its version goes up (a tensor saved for backward that was overwritten
+    is an error, not a wrong gradient), a leaf that requires grad is refused, gradients pass through."""
+    x = torch.ones(1000, device="cuda")
+    for fn in _collectives():
+        a = torch.full((1000,), 3.0, device="cuda", requires_grad=True)
+        b = a * 2
+        y = (b * b).sum()
+        version = b._version
+        with torch.no_grad():
+            fn(comm, x, b)
+        assert b._version > version and torch.equal(b, x)
+        with pytest.raises(RuntimeError, match="inplace operation"):
+            y.backward()
+        if fn.__name__ != "all_gather":        # (that one stores through a view of the bytes, which autograd does not follow)
+            with pytest.raises(RuntimeError):
+                fn(comm, x, a)
+            assert bool((a == 3.0).all())
+        with torch.no_grad():
+            fn(comm, x, a)
+        assert torch.equal(a.detach(), x)
+        with torch.inference_mode():
+            frozen = torch.zeros(1000, device="cuda")
+            fn(comm, x, frozen)
+            assert torch.equal(frozen, x)
+        if fn.__name__ != "all_gather":
+            with pytest.raises(RuntimeError, match="[Ii]nference"):
+                fn(comm, x, frozen)
+    from mccs_b200 import ops
+    w = torch.ones(1000, device="cuda", requires_grad=True)
+    out = torch.zeros(1000, device="cuda")
+    (ops.all_reduce(comm, w * 5, out) * 2).sum().backward()
+    assert torch.equal(w.grad, torch.full_like(w, 10.0))
