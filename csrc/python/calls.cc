@@ -317,6 +317,9 @@ PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   int dtype;
   const bool service = g_mem_info(from, nullptr, nullptr, nullptr) == mccsSuccess && g_mem_info(to, nullptr, nullptr, nullptr) == mccsSuccess;
   if (service ? !known_type(*in, &dtype) : autograd_takes_part(*in, *out)) Py_RETURN_FALSE;
+  // The tensors belong to the current stream's order, whichever stream the collective is given: the staged
+  // form copies there.
+  if (!service && stream != (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()) Py_RETURN_FALSE;
   mccsResult_t rc;
   const mccsComm_t comm = self->comm;
   Py_BEGIN_ALLOW_THREADS

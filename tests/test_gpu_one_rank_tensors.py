@@ -189,3 +189,18 @@ def test_autograd_sees_the_write(comm):
     out = torch.zeros(1000, device="cuda")
     (ops.all_reduce(comm, w * 5, out) * 2).sum().backward()
     assert torch.equal(w.grad, torch.full_like(w, 10.0))
+
+
+def test_a_collective_given_another_stream(comm):
+    """Input and output stay in the order of the current stream, however far behind the named one is."""
+    side = torch.cuda.Stream()
+    for it, fn in enumerate(_collectives()):
+        recv = torch.zeros(1 << 20, device="cuda")
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)          # about 10 ms
+        send = torch.full((1 << 20,), float(it + 1), device="cuda")
+        fn(comm, send, recv, stream=side)
+        seen = recv.clone()
+        send.fill_(-1.0)
+        torch.cuda.synchronize()
+        assert bool((seen == float(it + 1)).all()) and torch.equal(recv, seen), fn.__name__
