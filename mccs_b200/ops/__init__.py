@@ -94,6 +94,14 @@ def arena(comm: Communicator) -> _Arena:
     return a
 
 
+def _copied(comm: Communicator, send: torch.Tensor, out: torch.Tensor, op: str, algo: str, stream) -> bool:
+    """A communicator of one rank: whether ``out`` has been given ``send``'s values by one copy."""
+    if comm.nranks != 1 or OPS[op.lower()] == _PREMULSUM:
+        return False
+    ALGOS[algo]      # no kernel to choose, but an unknown name is an error with any number of ranks
+    return comm._calls.self_copy(send, out, stream)
+
+
 def all_reduce(comm: Communicator, send: torch.Tensor, recv: Optional[torch.Tensor] = None, *, op: str = "sum",
                scale: float = 1.0, algo: str = "auto", stream=None) -> torch.Tensor:
     """AllReduce of ``send`` into ``recv`` (in place when ``recv`` is None) over ``comm``.
@@ -106,7 +114,7 @@ def all_reduce(comm: Communicator, send: torch.Tensor, recv: Optional[torch.Tens
     out = send if recv is None else recv
     if send.numel() == 0:
         return out
-    if comm.nranks == 1 and OPS[op.lower()] != _PREMULSUM and comm._calls.self_copy(send, out, stream):
+    if _copied(comm, send, out, op, algo, stream):
         return out
     if usable_in_place(send) and (recv is None or usable_in_place(recv)):
         comm.all_reduce(send, recv, op=op, scale=scale, algo=algo, stream=stream)
@@ -130,7 +138,7 @@ def all_gather(comm: Communicator, send: torch.Tensor, recv: torch.Tensor, *, al
     nb = send.numel() * send.element_size()
     if nb == 0:
         return recv
-    if comm.nranks == 1 and comm._calls.self_copy(send, recv, stream):
+    if _copied(comm, send, recv, "sum", algo, stream):
         return recv
     if usable_in_place(recv) and send.is_contiguous() and in_service_memory(send):
         comm.all_gather(send, recv, nbytes=nb, algo=algo, stream=stream)
@@ -156,7 +164,7 @@ def reduce_scatter(comm: Communicator, send: torch.Tensor, recv: torch.Tensor, *
     Staged like :func:`all_reduce` when a tensor is not in service memory."""
     if recv.numel() == 0:
         return recv
-    if comm.nranks == 1 and OPS[op.lower()] != _PREMULSUM and comm._calls.self_copy(send, recv, stream):
+    if _copied(comm, send, recv, op, algo, stream):
         return recv
     if usable_in_place(send) and usable_in_place(recv):
         comm.reduce_scatter(send, recv, op=op, scale=scale, algo=algo, stream=stream)

@@ -204,3 +204,16 @@ def test_a_collective_given_another_stream(comm):
         send.fill_(-1.0)
         torch.cuda.synchronize()
         assert bool((seen == float(it + 1)).all()) and torch.equal(recv, seen), fn.__name__
+
+
+def test_unknown_names_are_refused(comm):
+    from mccs_b200 import ops
+    x, y = torch.ones(8, device="cuda"), torch.zeros(8, device="cuda")
+    for fn in _collectives():
+        with pytest.raises(KeyError):
+            fn(comm, x, y, algo="no_such_kernel")
+    for fn in (ops.all_reduce, ops.reduce_scatter):
+        with pytest.raises(KeyError):
+            fn(comm, x, y, op="no_such_operator")
+    torch.cuda.synchronize()
+    assert not bool(y.any())
