@@ -16,6 +16,7 @@
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/InferenceMode.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda.h>
 #include <dlfcn.h>
@@ -431,8 +432,8 @@ PyObject* local_all_reduce(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Py_DECREF(seq[0]);
   Py_DECREF(seq[1]);
   if (bad) { PyErr_SetString(PyExc_ValueError, bad); return nullptr; }
-  CUdevice now = -1;
-  if (!g_ctx_device || g_ctx_device(&now) != CUDA_SUCCESS || (int)now != device) Py_RETURN_NONE;
+  // (The runtime's device: a thread that has not used CUDA yet has one, but no context of the driver's.)
+  if ((int)c10::cuda::current_device() != device) Py_RETURN_NONE;
   uint64_t stream = 0;
   if (args[3] == Py_None) {
     stream = (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();

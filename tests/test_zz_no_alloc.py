@@ -160,3 +160,14 @@ def test_ops_binding_of_the_no_alloc_entry(service):
         ops.local_all_reduce_no_alloc([torch.zeros(4, device="cuda", dtype=torch.int32)])
     with pytest.raises(ValueError):
         ops.local_all_reduce_no_alloc([torch.zeros(4, device="cuda"), torch.zeros(5, device="cuda")])
+
+
+def test_ops_binding_from_a_thread_that_has_not_used_cuda(service):
+    """A new thread has no CUDA context current until its first launch; the call is that launch."""
+    from mccs_b200 import ops
+    torch.cuda.set_device(0)
+    xs = [torch.full((1000,), float(r + 1), device="cuda") for r in range(3)]
+    torch.cuda.synchronize()
+    run_ranks(1, lambda r: ops.local_all_reduce_no_alloc(xs))
+    torch.cuda.synchronize()
+    assert all(bool((x == 6.0).all()) for x in xs)
