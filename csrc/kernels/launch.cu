@@ -103,6 +103,8 @@ const void* one_gpu_function(int kind, int dtype, int op, int nranks, bool ragge
   return nullptr;
 }
 
+const void* local_copy_function(bool ragged) { return ragged ? mccs_kfn_local_copy_ragged() : mccs_kfn_untyped(kLocalCopy); }
+
 static int cooperative_fit(const void* fn, int threads, int nranks) {
   if (!fn || nranks <= 0) return 0;
   int dev = 0, sms = 0, per_sm = 0;
@@ -167,8 +169,8 @@ static OneGpuTile one_gpu_tile(int kind, int n, bool ragged, uint64_t packs) {
                                                : (n <= 4 ? kReduceUnrollFew : 1);
   // 128 threads measured as fast as or faster than 256, as long as a CTA moves 16 KiB: the GPU
   // starts one CTA in about 2.7 ns, so smaller ones cannot keep up with the memory. The reduction
-  // over more than four ranks needs the larger CTA for large messages (eight ranks, 200 MiB
-  // blocks scattered: 273 us against 352 us) but not for a few waves, where what counts is how
+  // over more than four ranks needs the larger CTA for large messages (eight ranks scattering
+  // 200 MiB each in blocks of 25 MiB: 273 us against 352 us) but not for a few waves, where what counts is how
   // evenly the last CTAs end. The shortest messages are spread until every SM has a CTA.
   const uint64_t buffers = (kind == kAllGather ? 1 : (uint64_t)n) + (kind == kReduceScatter ? 1 : (uint64_t)n);
   uint64_t threads = 128;
@@ -297,8 +299,10 @@ cudaError_t launch_collective(int kind, const CollArgs& args, LaunchDims dims, v
   dim3 grid((unsigned)dims.ctas, a.emulated ? (unsigned)a.nranks : 1u, 1u);
   dim3 block((unsigned)dims.threads, 1u, 1u);
   void* params[] = {(void*)&a};
-  if (a.variant == kLocalCopy && (((uint64_t)a.send[a.rank] | (uint64_t)a.recv[a.rank]) & 15u) != 0) fn = mccs_kfn_local_copy_ragged();
-  if (a.variant == kLocalCopy) return launch_local(fn, grid, block, params, stream);
+  if (a.variant == kLocalCopy) {
+    fn = local_copy_function((((uint64_t)a.send[a.rank] | (uint64_t)a.recv[a.rank]) & 15u) != 0);
+    return launch_local(fn, grid, block, params, stream);
+  }
   if (a.emulated && a.nranks > 1) {
     // All ranks' CTAs wait on one another, so they must be resident together.
     return cudaLaunchCooperativeKernel(fn, grid, block, params, 0, (cudaStream_t)stream);

@@ -22,6 +22,8 @@ int max_cooperative_ctas(int variant, int dtype, int op, int threads, int nranks
 cudaError_t launch_one_gpu(int kind, const CollArgs& args, int max_ctas, bool completion, void* stream);
 // The kernel such a launch runs; null when there is none for this type and operator.
 const void* one_gpu_function(int kind, int dtype, int op, int nranks, bool ragged, bool batch = false);
+// The copy of a communicator of one rank; `ragged`: not both buffers are 16-byte aligned.
+const void* local_copy_function(bool ragged);
 // Several such collectives in one launch, with a completion word (b.base.seq).
 cudaError_t launch_one_gpu_batch(const BatchArgs& b, void* stream);
 

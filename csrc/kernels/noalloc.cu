@@ -38,7 +38,11 @@ extern "C" int mccsLocalAllReduceNoAllocPrepare(void) {
         cudaError_t e = load(one_gpu_function(kAllReduce, dt, kSum, n, ragged));
         if (e != cudaSuccess) return (int)e;
       }
-  return (int)load(kernel_function(kLocalCopy, kFloat32, kSum));
+  for (bool ragged : {false, true}) {   // one buffer: a copy
+    cudaError_t e = load(local_copy_function(ragged));
+    if (e != cudaSuccess) return (int)e;
+  }
+  return (int)cudaSuccess;
 }
 
 extern "C" int mccsLocalAllReduceNoAllocStatus(mccsNoAllocStatus_t* status, void* stream) {
