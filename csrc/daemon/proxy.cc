@@ -970,23 +970,32 @@ void ProxyEngine::begin_group(Communicator& c, CollSlot& s, uint64_t seq, void* 
   order_after_last_launch(c, stream);
 }
 
-// ... and the callers' streams behind the kernel: at once, or through what the client waits for.
+// ... and the callers' streams behind the kernel, those of every member: at once, or through what the
+// client waits for.
 void ProxyEngine::end_group(Communicator& c, CollSlot& s, uint64_t seq, void* stream) {
   Backend* be = daemon_->backend();
+  const int len = s.fused_kernel ? s.batch_len : 1;
   bool marked = false;
   for (int r = 0; r < c.nranks; r++) {
-    const CollOp& op = s.ops[r];
     RankState& rr = *c.ranks[(size_t)r];
-    if (op.on_caller_stream) {
-      if (op.caller_stream == stream) continue;
-      if (!marked) be->event_record(rr.device, c.mark_event, stream);
-      marked = true;
-      be->stream_wait_event(rr.device, op.caller_stream, c.mark_event);
-    } else if (rr.sync.host && op.sync_slot) {
-      be->stream_write_value64(rr.device, stream, rr.sync.dev_addr + 8 * proto::kSyncDoneSlot,
-                               s.fused_kernel ? last_member_user_seq(c, s, seq, r) : op.user_seq);
-    } else {
-      be->event_record(rr.device, rr.backend_event, stream);
+    void* released = stream;   // the stream that has just been seen to
+    bool answered = false;
+    for (int k = 0; k < len; k++) {
+      const CollOp& op = (k == 0 ? s : c.slot(seq + (uint64_t)k)).ops[r];
+      if (op.on_caller_stream) {
+        if (op.caller_stream == stream || op.caller_stream == released) continue;
+        if (!marked) be->event_record(rr.device, c.mark_event, stream);
+        marked = true;
+        be->stream_wait_event(rr.device, op.caller_stream, c.mark_event);
+        released = op.caller_stream;
+      } else if (!answered) {
+        answered = true;   // one mark covers every member
+        if (rr.sync.host && op.sync_slot)
+          be->stream_write_value64(rr.device, stream, rr.sync.dev_addr + 8 * proto::kSyncDoneSlot,
+                                   s.fused_kernel ? last_member_user_seq(c, s, seq, r) : op.user_seq);
+        else
+          be->event_record(rr.device, rr.backend_event, stream);
+      }
     }
   }
 }

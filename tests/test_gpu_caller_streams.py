@@ -60,3 +60,59 @@ def test_collectives_are_ordered_with_the_callers_streams(service, n, mode):
         q = c.query()
         assert q["async_error"] == 0 and q["device_error"] == 0
         c.destroy()
+
+
+FUSED = r"""
+import os, threading
+import torch
+import mccs_b200 as M
+
+torch.cuda.set_device(0)
+M.init(M.daemon.start_embedded(prefix=f"/tmp/mccs-fused-streams-{os.getpid()}", listen_port=-1, extra="fuse_allreduce = 4"))
+n, count, comms = 2, 1 << 20, [None, None]
+ts = [threading.Thread(target=lambda r=r: comms.__setitem__(r, M.Communicator(41, r, n, device=0))) for r in range(n)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+bufs = [M.Buffer(count * 4, 0) for _ in range(4 * n)]
+a, ra, b, rb = ([x.tensor(torch.float32, count) for x in bufs[i::4]] for i in range(4))
+s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+for it in range(6):
+    for r in range(n):
+        a[r].fill_(float(it + r)); b[r].fill_(float(10 * it + r)); ra[r].fill_(-1.0); rb[r].fill_(-1.0)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s1):
+        torch.cuda._sleep(20_000_000)        # the launch cannot run before this has ended
+    # held back until the whole group waits: its two calls go out in one launch
+    assert M.daemon.embedded_admin({"cmd": "pause", "communicator_id": 41})["status"] == "ok"
+    threading.Timer(0.1, lambda: M.daemon.embedded_admin({"cmd": "resume", "communicator_id": 41})).start()
+    with M.group():
+        for r in range(n):
+            comms[r].all_reduce(a[r], ra[r], algo="ar_twoshot", stream=s1)
+        for r in range(n):
+            comms[r].all_reduce(b[r], rb[r], algo="ar_twoshot", stream=s2)
+    seen = []
+    for stream, out, want in ((s1, ra, 2 * it + 1), (s2, rb, 20 * it + 1)):
+        with torch.cuda.stream(stream):
+            seen += [(x.clone(), float(want)) for x in out]
+    torch.cuda.synchronize()
+    for k, (x, want) in enumerate(seen):
+        assert bool((x == want).all()), (it, k, x[:4].tolist(), want)
+stats = M.daemon.embedded_admin({"cmd": "stats"})["stats"]["communicators"]["41"]
+assert stats["fused_members"] == 12, stats
+for c in comms:
+    c.destroy()
+M.finalize()
+M.daemon.stop_embedded()
+print("OK")
+"""
+
+
+def test_members_of_a_fused_launch_on_streams_of_their_own():
+    """With ``fuse_allreduce`` one launch carries calls that were given different streams: each of them waits for it."""
+    import os
+    import subprocess
+    import sys
+
+    from helpers import REPO
+    p = subprocess.run([sys.executable, "-c", FUSED], env=dict(os.environ, PYTHONPATH=REPO), capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and p.stdout.strip().endswith("OK"), p.stdout[-2000:] + p.stderr[-3000:]
