@@ -132,23 +132,32 @@ __device__ __forceinline__ void trace_begin(const CollArgs& a, int rank) {
 // while another CTA of the rank is still storing: each CTA's closing barrier only covers
 // the CTAs with its own index on the peers. The CTAs therefore count themselves off and
 // the last one publishes the word.
-// kLocal: everything the kernel wrote is memory of this GPU, so ordering at GPU scope before the
-// counts is enough and the word is a plain store behind the last one (the system-scope fence and
-// release store make a launch about 3 us longer).
-template <bool kLocal = false>
 __device__ __forceinline__ void finish(const CollArgs& a, int rank) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();   // this CTA's stores are ordered before its count
     const unsigned last = gridDim.x - 1;
     if (atomicInc(&a.pad[rank]->pad_[kPadCtaCounter], last) == last) {
-      if (kLocal && !a.trace) {
-        st_relaxed_sys_u64(&a.status[rank]->done_seq, a.seq);
-        return;
-      }
       fence_sys();     // ... and, through the counts, before the completion word
       if (a.trace) st_relaxed_sys_u64(&a.status[rank]->end_ns, globaltimer_ns());
       st_release_sys_u64(&a.status[rank]->done_seq, a.seq);
+    }
+  }
+}
+
+// The same for a kernel that only wrote memory of this GPU: order at GPU scope, which the counts carry, is
+// enough and the word is a plain store (the system-scope fence and release store make a launch about 3 us
+// longer).
+__device__ __forceinline__ void finish_local(const CollArgs& a, int rank) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned last = gridDim.x - 1;
+    if (count_off(&a.pad[rank]->pad_[kPadCtaCounter], last) == last) {
+      if (a.trace) {
+        st_relaxed_sys_u64(&a.status[rank]->end_ns, globaltimer_ns());
+        fence_sys();   // whoever reads the word finds the time
+      }
+      st_relaxed_sys_u64(&a.status[rank]->done_seq, a.seq);
     }
   }
 }
@@ -666,7 +675,7 @@ __global__ void __launch_bounds__(kMaxThreads) local_copy_kernel(const __grid_co
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = done + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < bytes; i += stride) out[i] = in[i];
   }
-  if (a.pad[rank] != nullptr) finish<true>(a, rank);   // no completion word for callers without a communicator
+  if (a.pad[rank] != nullptr) finish_local(a, rank);   // no completion word for callers without a communicator
 }
 
 // The same for buffers that are not both 16-byte aligned: the packs are aligned in the output, the
@@ -699,7 +708,7 @@ __global__ void __launch_bounds__(kMaxThreads) local_copy_ragged_kernel(const __
       out[k] = in[k];
     }
   }
-  if (a.pad[a.rank] != nullptr) finish<true>(a, a.rank);
+  if (a.pad[a.rank] != nullptr) finish_local(a, a.rank);
 }
 
 #endif  // MCCS_UNTYPED_KERNELS

@@ -66,6 +66,14 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 __device__ __forceinline__ void fence_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
+// Counts up to `last` and wraps to zero; returns the count found. Orders, at GPU scope, what the CTA did
+// before (its other threads through the barrier in front) ahead of the count, and what the CTAs counted
+// before did ahead of whatever follows: one instruction in place of a fence on either side of the count.
+__device__ __forceinline__ uint32_t count_off(uint32_t* counter, uint32_t last) {
+  uint32_t found;
+  asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(found) : "l"(counter), "r"(last) : "memory");
+  return found;
+}
 
 // ----------------------------------------------------------------------------
 // Bulk data loads/stores. Peer memory is read with system-scope relaxed loads so

@@ -32,16 +32,15 @@ namespace mccs {
 namespace dev {
 
 // Completion word of the launch, as finish() in collectives.cuh, for the whole grid at once.
-// Everything the kernel wrote is memory of this GPU, so ordering the CTAs' stores at GPU scope
-// before the count is enough; the word itself is a plain store to host memory behind the last
-// count. (A system-scope fence in front of it and a release store made every launch 3 us longer.)
+// Everything the kernel wrote is memory of this GPU, so order at GPU scope is enough: the counts carry it
+// from every CTA's stores to the last CTA, whose word is then a plain store to host memory. (A
+// system-scope fence in front of it and a release store made every launch 3 us longer.)
 __device__ __forceinline__ void one_gpu_finish(const OneGpuArgs& a) {
   if (a.counter == nullptr) return;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
     const unsigned last = gridDim.x * gridDim.y - 1;
-    if (atomicInc(a.counter, last) == last) {
+    if (count_off(a.counter, last) == last) {
       if (a.trace) {
         const uint64_t t = globaltimer_ns();
         for (int r = 0; r < a.nranks; r++) st_relaxed_sys_u64(&a.status[r]->end_ns, t);

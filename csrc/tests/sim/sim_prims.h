@@ -22,6 +22,7 @@ inline void st_release_sys_u64(uint64_t* p, uint64_t v) { __atomic_store_n(p, v,
 inline void st_relaxed_sys_u64(uint64_t* p, uint64_t v) { __atomic_store_n(p, v, __ATOMIC_SEQ_CST); }
 inline uint64_t globaltimer_ns() { return sim::now_ns(); }
 inline void fence_sys() { __atomic_thread_fence(__ATOMIC_SEQ_CST); }
+inline uint32_t count_off(uint32_t* counter, uint32_t last) { return atomicInc(counter, last); }
 
 template <int BYTES> struct Raw;
 template <> struct Raw<1> { uint8_t x; };
