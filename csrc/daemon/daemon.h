@@ -188,7 +188,7 @@ class Communicator {
   // Clients inside the daemon's process, one GPU: kernels go to the callers' streams. Which
   // stream the newest kernel went to, and an event for callers on different streams.
   bool caller_streams = false;
-  void* last_stream = nullptr;
+  uint64_t last_stream_id = 0;    // (0: not known)
   void* mark_event = nullptr;
 
   CollSlot slots[kCollSlots];

@@ -926,16 +926,19 @@ void ProxyEngine::signal_done(RankState& rs, uint64_t user_seq, int status) {
 
 // Clients inside the daemon's process on one GPU. Collectives of a communicator run in order
 // whatever streams their callers use (its kernels share a counter, and done_seq only grows); on
-// one stream that is given, after a change of stream the new one waits for the last kernel. That
+// one stream that is given, after a change of stream (told by its id: a destroyed stream's handle may be
+// another stream's by now, its kernel still queued) the new one waits for the last kernel. That
 // wait can only ever sit behind the kernel it waits for, also in a hardware queue that both
 // streams share: the kernel was launched before.
 void ProxyEngine::order_after_last_launch(Communicator& c, void* stream) {
   if (!c.caller_streams) return;
   const RankState& r0 = *c.ranks[0];
   const uint64_t ticket = r0.last_ticket.load(std::memory_order_relaxed);
-  if (c.last_stream != stream && ticket > __atomic_load_n(&r0.status->done_seq, __ATOMIC_ACQUIRE))
+  uint64_t id = 0;
+  if (daemon_->backend()->stream_id(r0.device, stream, &id) != proto::kOk) id = 0;
+  if ((id == 0 || id != c.last_stream_id) && ticket > __atomic_load_n(&r0.status->done_seq, __ATOMIC_ACQUIRE))
     daemon_->backend()->stream_wait_value64(r0.device, stream, (uint64_t)&r0.status->done_seq, ticket);
-  c.last_stream = stream;
+  c.last_stream_id = id;
 }
 
 // The stream a launch for all ranks goes to: the caller's, when every rank's caller is on the

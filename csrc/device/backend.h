@@ -106,6 +106,9 @@ class Backend {
   virtual int stream_destroy(int dev, void* stream) = 0;
   virtual int stream_query(int dev, void* stream) = 0;   // 0 idle, 1 busy, <0 Status
   virtual int stream_sync(int dev, void* stream) = 0;
+  // A number no other stream of this process has or will have (a handle is given out again after
+  // its stream was destroyed, with work still queued perhaps).
+  virtual int stream_id(int dev, void* stream, uint64_t* id) = 0;
   virtual int event_create(int dev, void** ev, uint8_t handle[proto::kIpcHandleBytes]) = 0;
   virtual int event_open(int dev, const uint8_t handle[proto::kIpcHandleBytes], void** ev) = 0;
   virtual int event_destroy(int dev, void* ev) = 0;

@@ -377,6 +377,17 @@ class CudaBackend : public Backend {
     cudaStreamDestroy((cudaStream_t)stream);
     return proto::kOk;
   }
+  int stream_id(int, void* stream, uint64_t* id) override {
+    unsigned long long v = 0;
+    cudaError_t e = cudaStreamGetId((cudaStream_t)stream, &v);
+    if (e != cudaSuccess) {
+      LOG_ERROR("cudaStreamGetId: %s", cudaGetErrorString(e));
+      cudaGetLastError();
+      return proto::kErrDevice;
+    }
+    *id = v;
+    return proto::kOk;
+  }
   int stream_query(int, void* stream) override {
     cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
     if (e == cudaSuccess) return 0;

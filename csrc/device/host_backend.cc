@@ -247,6 +247,7 @@ class HostBackend : public Backend {
   int stream_destroy(int, void*) override { return proto::kOk; }
   int stream_query(int, void*) override { return 0; }
   int stream_sync(int, void*) override { return proto::kOk; }
+  int stream_id(int, void* stream, uint64_t* id) override { *id = (uint64_t)stream; return proto::kOk; }
   int event_create(int, void** ev, uint8_t handle[proto::kIpcHandleBytes]) override {
     *ev = (void*)(uintptr_t)(++next_handle_);
     memset(handle, 0, proto::kIpcHandleBytes);

@@ -235,7 +235,6 @@ struct mccsComm {
   bool caller_streams = false;
   const uint64_t* done_seq = nullptr;
   uint64_t last_ticket = 0;
-  mccsStream_t last_stream = nullptr;   // where the newest of those collectives went
   bool deferred_wait = false;         // collectives do not queue "wait done"; mccsCommWait does
   uint64_t last_posted_seq = 0;       // user_seq of the newest request posted
   pthread_t owner = pthread_self();   // the thread that created (and uses) the communicator
@@ -1210,7 +1209,6 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
   if (on_caller_stream) {
     wr.flags |= proto::kWrCallerStream;
     wr.caller_stream = (uint64_t)stream;
-    comm->last_stream = stream;
   } else if (g_ctx.backend == proto::kBackendCuda) {
     CtxScope scope(comm->device);
     if (!scope.ok) return mccsDeviceError;
@@ -1792,10 +1790,11 @@ mccsResult_t mccsCommWait(mccsComm_t comm, mccsStream_t stream) {
     // "done" only grows and is written in submission order: the newest value covers all.
     return sem_wait_geq(comm, stream, comm->sync_base + 8 * proto::kSyncDoneSlot, comm->last_posted_seq);
   }
-  if (comm->caller_streams && comm->last_ticket && comm->last_stream != stream &&
+  if (comm->caller_streams && comm->last_ticket &&
       __atomic_load_n(comm->done_seq, __ATOMIC_ACQUIRE) < comm->last_ticket) {
     // Collectives of a communicator end in order, so the newest ticket covers all of them. The
-    // kernel that raises the word has been launched already (the ticket came with the completion).
+    // kernel that raises the word has been launched already (the ticket came with the completion), on
+    // `stream` itself perhaps: then the wait ends where it starts.
     CtxScope scope(comm->device);
     if (!scope.ok) return mccsDeviceError;
     mccsResult_t r = sem_wait_geq(comm, stream, (uint64_t)comm->done_seq, comm->last_ticket);

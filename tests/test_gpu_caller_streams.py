@@ -8,7 +8,7 @@ import threading
 import pytest
 import torch
 
-from helpers import fresh_comm_id
+from helpers import fresh_comm_id, run_ranks
 
 pytestmark = pytest.mark.gpu
 
@@ -116,3 +116,56 @@ def test_members_of_a_fused_launch_on_streams_of_their_own():
     from helpers import REPO
     p = subprocess.run([sys.executable, "-c", FUSED], env=dict(os.environ, PYTHONPATH=REPO), capture_output=True, text=True, timeout=300)
     assert p.returncode == 0 and p.stdout.strip().endswith("OK"), p.stdout[-2000:] + p.stderr[-3000:]
+
+
+@pytest.mark.parametrize("n", [1, 2])
+def test_streams_destroyed_while_their_collective_waits(service, n):
+    """A stream may be destroyed while work is queued on it, and its handle given to the next one: the next
+    collective and whoever waits for the communicator are still behind the old stream's."""
+    import ctypes
+    M, count, cid, comms = service, 1 << 20, fresh_comm_id(), [None] * n
+    torch.cuda.set_device(0)
+    run_ranks(n, lambda r: comms.__setitem__(r, M.Communicator(cid, r, n, device=0)))
+    bufs = [M.Buffer(count * 4, 0) for _ in range(3 * n)]
+    x, y, z = ([b.tensor(torch.float32, count) for b in bufs[i::3]] for i in range(3))
+    lib, other, handles = ctypes.CDLL("libcuda.so.1"), torch.cuda.Stream(), []
+
+    def create():
+        s = ctypes.c_void_p()
+        assert lib.cuStreamCreate(ctypes.byref(s), 1) == 0
+        handles.append(s.value)
+        return s, torch.cuda.ExternalStream(s.value)
+
+    def reduce(src, dst, stream):
+        with M.group():
+            for r in range(n):
+                comms[r].all_reduce(src[r], dst[r], stream=stream)
+
+    for it in range(12):
+        for r in range(n):
+            y[r].fill_(-1.0)
+            z[r].fill_(-1.0)
+        torch.cuda.synchronize()
+        old, stream = create()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(10_000_000)
+            for r in range(n):
+                x[r].fill_(float(it + r))
+        reduce(x, y, stream)
+        assert lib.cuStreamDestroy_v2(old) == 0
+        new, stream = create()
+        if it % 2:
+            reduce(y, z, stream)
+            with torch.cuda.stream(stream):
+                seen = [t.clone() for t in z]
+        else:
+            comms[0].wait(stream)
+            with torch.cuda.stream(stream):
+                seen = [t.clone() for t in y]
+        torch.cuda.synchronize()
+        want = float(n * it + n * (n - 1) // 2) * (n if it % 2 else 1)
+        assert all(bool((t == want).all()) for t in seen), (it, want, seen[0][:4].tolist())
+        assert lib.cuStreamDestroy_v2(new) == 0
+    print(f"{len(handles) - len(set(handles))} of {len(handles)} handles were given out again")
+    for c in comms:
+        c.destroy()
