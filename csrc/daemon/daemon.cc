@@ -333,18 +333,26 @@ void Daemon::on_malloc(Session& s, const proto::MallocReq& m) {
   reply(s, r, sizeof(proto::MallocReply), send_fd ? &a.share_fd : nullptr, send_fd ? 1 : 0);
 }
 
-// Kernels on the callers' own streams: the daemon waits for the completion word of the newest
-// one instead of a stream (whose handle is not its own). Every one of them ends, or has reported
-// an error; the bound is for a GPU that has stopped.
-void Daemon::wait_for_caller_streams(Communicator& c) {
-  if (!c.caller_streams || !c.ranks[0] || !c.ranks[0]->status) return;
-  const StatusBlock* st = c.ranks[0]->status;
-  const uint64_t ticket = c.ranks[0]->last_ticket.load(std::memory_order_relaxed);
-  const uint64_t t_end = monotonic_us() + 60ull * 1000 * 1000;
-  while (__atomic_load_n(&st->done_seq, __ATOMIC_ACQUIRE) < ticket && __atomic_load_n(&st->error, __ATOMIC_ACQUIRE) == kDevOk &&
-         monotonic_us() < t_end) {
+void wait_for_done_seq(const StatusBlock* st, uint64_t ticket, const std::function<bool()>& alive) {
+  for (unsigned round = 1; __atomic_load_n(&st->done_seq, __ATOMIC_ACQUIRE) < ticket; round++) {
+    if (round % 64 == 0 && !alive()) return;
     struct timespec ts = {0, 20000};
     nanosleep(&ts, nullptr);
+  }
+}
+
+// Kernels on the callers' own streams: the daemon waits for the newest one's completion word, or for the
+// event behind a kernel that may end without it, instead of a stream (whose handle is not its own). Like
+// the synchronisation of a stream this ends with the kernel.
+void Daemon::wait_for_caller_streams(Communicator& c) {
+  if (!c.caller_streams || !c.ranks[0] || !c.ranks[0]->status || !c.ranks[0]->stream) return;
+  RankState& r0 = *c.ranks[0];
+  const uint64_t ticket = r0.last_ticket.load(std::memory_order_acquire);
+  if (c.newest_by_event.load(std::memory_order_acquire)) {
+    backend_->stream_wait_event(r0.device, r0.stream, r0.backend_event);
+    backend_->stream_sync(r0.device, r0.stream);
+  } else {
+    wait_for_done_seq(r0.status, ticket, [&] { return backend_->stream_query(r0.device, r0.stream) >= 0; });
   }
 }
 

@@ -20,6 +20,7 @@
 #pragma once
 #include <atomic>
 #include <deque>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -166,6 +167,11 @@ struct RankState {
 
 enum CommState : int { kCommInit = 0, kCommActive = 1, kCommError = 2, kCommClosed = 3 };
 
+// Returns once the word at `st` has reached `ticket`, whatever error the block shows meanwhile (later kernels
+// still run), or the GPU has stopped (`alive` says so; asked about every millisecond). A kernel on a
+// caller's stream may sit behind other work of the caller's for any time.
+void wait_for_done_seq(const StatusBlock* st, uint64_t ticket, const std::function<bool()>& alive);
+
 class Communicator {
  public:
   uint32_t id = 0;
@@ -189,6 +195,9 @@ class Communicator {
   // stream the newest kernel went to, and an event for callers on different streams.
   bool caller_streams = false;
   uint64_t last_stream_id = 0;    // (0: not known)
+  // Whether the newest kernel may end without its completion word (it gives up when a wait runs out): then
+  // rank 0's backend event is recorded behind it.
+  std::atomic<bool> newest_by_event{false};
   void* mark_event = nullptr;
 
   CollSlot slots[kCollSlots];
@@ -256,6 +265,7 @@ class ProxyEngine : public Engine {
   bool publish_plan_error(RankState& rs, uint64_t user_seq, int status);
   void order_after_client(RankState& rs, const CollOp& op, void* stream);
   void order_after_last_launch(Communicator& c, void* stream);
+  void note_launch(Communicator& c, int variant, void* stream);
   void* stream_for_group(Communicator& c, CollSlot& s, uint64_t seq);
   void begin_group(Communicator& c, CollSlot& s, uint64_t seq, void* stream);
   void end_group(Communicator& c, CollSlot& s, uint64_t seq, void* stream);

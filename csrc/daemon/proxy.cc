@@ -866,7 +866,8 @@ bool ProxyEngine::launch_slices(RankState& rs, CollSlot& s, uint64_t seq) {
       const uint64_t bytes = s.nslices == 1 ? s.plan.bytes : s.plan.bytes / (uint64_t)s.nslices;
       rs.inflight.push_back({a.seq, bytes});
     }
-    rs.last_ticket.store(a.seq, std::memory_order_relaxed);
+    note_launch(c, s.plan.variant, stream);
+    rs.last_ticket.store(a.seq, std::memory_order_release);
     rs.next_slice++;
   }
   if (op.on_caller_stream)
@@ -936,9 +937,22 @@ void ProxyEngine::order_after_last_launch(Communicator& c, void* stream) {
   const uint64_t ticket = r0.last_ticket.load(std::memory_order_relaxed);
   uint64_t id = 0;
   if (daemon_->backend()->stream_id(r0.device, stream, &id) != proto::kOk) id = 0;
-  if ((id == 0 || id != c.last_stream_id) && ticket > __atomic_load_n(&r0.status->done_seq, __ATOMIC_ACQUIRE))
-    daemon_->backend()->stream_wait_value64(r0.device, stream, (uint64_t)&r0.status->done_seq, ticket);
+  if ((id == 0 || id != c.last_stream_id) && ticket > __atomic_load_n(&r0.status->done_seq, __ATOMIC_ACQUIRE)) {
+    if (c.newest_by_event.load(std::memory_order_relaxed)) daemon_->backend()->stream_wait_event(r0.device, stream, r0.backend_event);
+    else daemon_->backend()->stream_wait_value64(r0.device, stream, (uint64_t)&r0.status->done_seq, ticket);
+  }
   c.last_stream_id = id;
+}
+
+// A launch for callers in this process has been made. Behind a kernel that may give up without its
+// completion word every rank's event is recorded, for whoever waits for it: the next stream, the clients
+// (mccsCommWait), the release of memory.
+void ProxyEngine::note_launch(Communicator& c, int variant, void* stream) {
+  if (!c.caller_streams) return;
+  const bool by_event = variant_waits(variant);
+  if (by_event)
+    for (auto& r : c.ranks) daemon_->backend()->event_record(r->device, r->backend_event, stream);
+  c.newest_by_event.store(by_event, std::memory_order_release);
 }
 
 // The stream a launch for all ranks goes to: the caller's, when every rank's caller is on the
@@ -1020,7 +1034,8 @@ bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
       c.state.store(kCommError);
     } else {
       r0.inflight.push_back({b.base.seq, s.batch_bytes, s.plan.variant == kOneGpu ? (uint64_t)s.batch_len : 1});
-      r0.last_ticket.store(b.base.seq, std::memory_order_relaxed);
+      note_launch(c, s.plan.variant, stream);
+      r0.last_ticket.store(b.base.seq, std::memory_order_release);
     }
     r0.next_slice = 1;
     end_group(c, s, seq, stream);
@@ -1040,7 +1055,8 @@ bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
     }
     const uint64_t bytes = s.nslices == 1 ? s.plan.bytes : s.plan.bytes / (uint64_t)s.nslices;
     r0.inflight.push_back({a.seq, bytes});
-    r0.last_ticket.store(a.seq, std::memory_order_relaxed);
+    note_launch(c, s.plan.variant, stream);
+    r0.last_ticket.store(a.seq, std::memory_order_release);
     r0.next_slice++;
   }
   end_group(c, s, seq, stream);

@@ -82,7 +82,8 @@ struct alignas(128) SignalPad {
   uint64_t ring_head[kMaxRingChannels];
   // Counters of finished CTAs of the owner's kernels (wrap to zero at the grid size, so
   // they need no reset between launches): [kPadBatchCounter] for the fused kernels'
-  // caller-visible completion word, [kPadCtaCounter] for StatusBlock::done_seq.
+  // caller-visible completion word, [kPadCtaCounter] for StatusBlock::done_seq, [kPadOneGpuCounter] (rank
+  // 0's) for the same word of the kOneGpu kernels: a kernel that gave up a wait leaves its count half way.
   uint32_t pad_[32];
 };
 // Launch shape of the single-rank copy kernel: every thread moves kCopyUnroll 16-byte
@@ -92,6 +93,7 @@ constexpr int kCopyUnroll = 4;
 constexpr uint64_t kCopyTileBytes = (uint64_t)kCopyThreads * kCopyUnroll * 16;
 constexpr int kPadBatchCounter = 0;
 constexpr int kPadCtaCounter = 1;
+constexpr int kPadOneGpuCounter = 2;
 
 // Per-rank status block in pinned, host-mapped memory: the host reads it without
 // synchronising the stream.
@@ -244,7 +246,8 @@ inline const char* variant_name(int v) {
 }
 
 inline bool variant_is_nvls(int v) { return v == kArNvlsOne || v == kArNvlsTwo || v == kAgNvls || v == kArHybrid || v == kRsNvls; }
-// Kernels whose CTAs never wait for one another: nothing has to be resident together.
+// Kernels whose CTAs never wait for one another: nothing has to be resident together, and they always
+// reach their end and write their completion word.
 inline bool variant_waits(int v) { return v != kLocalCopy && v != kOneGpu; }
 inline bool variant_is_ring(int v) { return v == kArRing || v == kAgRing; }
 

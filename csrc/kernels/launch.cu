@@ -196,7 +196,7 @@ static void one_gpu_common(int kind, const CollArgs& args, bool completion, OneG
   a->trace = args.trace;
   a->scale = args.scale;
   a->seq = args.seq;
-  a->counter = completion ? &args.pad[0]->pad_[kPadCtaCounter] : nullptr;
+  a->counter = completion ? &args.pad[0]->pad_[kPadOneGpuCounter] : nullptr;
 }
 
 // The runtime loads a kernel's code at its first use, which takes milliseconds. Whoever launches one

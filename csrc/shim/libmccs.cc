@@ -235,6 +235,7 @@ struct mccsComm {
   bool caller_streams = false;
   const uint64_t* done_seq = nullptr;
   uint64_t last_ticket = 0;
+  uint32_t last_ticket_variant = 0;   // the kernel that raises done_seq to it
   bool deferred_wait = false;         // collectives do not queue "wait done"; mccsCommWait does
   uint64_t last_posted_seq = 0;       // user_seq of the newest request posted
   pthread_t owner = pthread_self();   // the thread that created (and uses) the communicator
@@ -693,7 +694,7 @@ mccsResult_t wait_completion(mccsComm* comm, proto::WorkCompletion* wc) {
   comm->outstanding--;
   comm->last_variant = wc->variant;
   comm->last_ctas = wc->ctas;
-  if (wc->ticket) comm->last_ticket = wc->ticket;
+  if (wc->ticket) { comm->last_ticket = wc->ticket; comm->last_ticket_variant = wc->variant; }
   if (wc->status != 0 && comm->sticky_error == 0) comm->sticky_error = wc->status;
   return (mccsResult_t)wc->status;
 }
@@ -722,7 +723,7 @@ void reap_completions(mccsComm* comm) {
     comm->outstanding--;
     comm->last_variant = wc.variant;
     comm->last_ctas = wc.ctas;
-    if (wc.ticket) comm->last_ticket = wc.ticket;
+    if (wc.ticket) { comm->last_ticket = wc.ticket; comm->last_ticket_variant = wc.variant; }
     if (wc.status != 0 && comm->sticky_error == 0) comm->sticky_error = wc.status;
   }
 }
@@ -1220,7 +1221,7 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
     proto::WorkCompletion wc;
     if (comm->outstanding > 0 && comm->cq.try_pop(&wc)) {
       comm->outstanding--;
-      if (wc.ticket) comm->last_ticket = wc.ticket;
+      if (wc.ticket) { comm->last_ticket = wc.ticket; comm->last_ticket_variant = wc.variant; }
       if (wc.status != 0 && comm->sticky_error == 0) comm->sticky_error = wc.status;
     }
   }
@@ -1790,11 +1791,12 @@ mccsResult_t mccsCommWait(mccsComm_t comm, mccsStream_t stream) {
     // "done" only grows and is written in submission order: the newest value covers all.
     return sem_wait_geq(comm, stream, comm->sync_base + 8 * proto::kSyncDoneSlot, comm->last_posted_seq);
   }
-  if (comm->caller_streams && comm->last_ticket &&
+  if (comm->caller_streams && comm->last_ticket && !variant_waits((int)comm->last_ticket_variant) &&
       __atomic_load_n(comm->done_seq, __ATOMIC_ACQUIRE) < comm->last_ticket) {
     // Collectives of a communicator end in order, so the newest ticket covers all of them. The
     // kernel that raises the word has been launched already (the ticket came with the completion), on
-    // `stream` itself perhaps: then the wait ends where it starts.
+    // `stream` itself perhaps: then the wait ends where it starts. (Behind a kernel that may give up without
+    // its word the daemon recorded the event below.)
     CtxScope scope(comm->device);
     if (!scope.ok) return mccsDeviceError;
     mccsResult_t r = sem_wait_geq(comm, stream, (uint64_t)comm->done_seq, comm->last_ticket);

@@ -14,6 +14,7 @@
 #include "../common/protocol.h"
 #include "../common/value.h"
 #include "../daemon/config.h"
+#include "../daemon/daemon.h"
 #include "../daemon/planner.h"
 #include "../daemon/qos.h"
 #include "../daemon/runtime.h"
@@ -597,6 +598,26 @@ static void test_qos_many_tenants() {
            (unsigned long long)asks.load());
 }
 
+// Memory a kernel on a caller's stream uses is kept until that kernel's word is there, also when an earlier
+// kernel has left an error, and no longer than the GPU runs.
+static void test_wait_for_done_seq() {
+  StatusBlock st;
+  memset(&st, 0, sizeof st);
+  st.error = kDevTimeoutStart;
+  st.done_seq = 3;
+  std::atomic<int> asked{0};
+  std::thread gpu([&] {
+    usleep(30000);
+    __atomic_store_n(&st.done_seq, (uint64_t)7, __ATOMIC_RELEASE);
+  });
+  wait_for_done_seq(&st, 7, [&] { asked++; return true; });
+  CHECK(__atomic_load_n(&st.done_seq, __ATOMIC_ACQUIRE) == 7 && asked > 0);
+  gpu.join();
+  wait_for_done_seq(&st, 7, [] { return false; });   // there already
+  wait_for_done_seq(&st, 8, [] { return false; });   // the GPU has stopped
+  CHECK(true);
+}
+
 static void test_misc() {
   std::vector<int> c = parse_cpu_list("0-3,8,10-11");
   CHECK(c.size() == 7 && c[4] == 8 && c[6] == 11);
@@ -620,6 +641,7 @@ int main() {
   test_ring_steps();
   test_qos();
   test_qos_many_tenants();
+  test_wait_for_done_seq();
   test_misc();
   printf("%d checks, %d failed\n", g_checks, g_failed);
   return g_failed;

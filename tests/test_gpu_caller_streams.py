@@ -62,6 +62,52 @@ def test_collectives_are_ordered_with_the_callers_streams(service, n, mode):
         c.destroy()
 
 
+def test_kernels_that_wait_for_one_another_on_callers_streams(service):
+    """The cooperative kernels may end without their completion word, so streams and the release of memory follow
+    an event behind them: mixed with the one-pass kernels on changing streams, read after
+    ``Communicator.wait`` elsewhere, and freed while queued (the free returns when the kernel has ended)."""
+    M, count, n = service, 1 << 18, 2
+    torch.cuda.set_device(0)
+    cid, comms = fresh_comm_id(), [None] * n
+    run_ranks(n, lambda r: comms.__setitem__(r, M.Communicator(cid, r, n, device=0)))
+    streams, other = [torch.cuda.Stream() for _ in range(2)], torch.cuda.Stream()
+    bufs = [M.Buffer(count * 4, 0) for _ in range(2 * n)]
+    x, y = ([b.tensor(torch.float32, count) for b in bufs[i::2]] for i in range(2))
+    for it, algo in enumerate(["ar_twoshot", "auto", "auto", "ar_twoshot", "ar_ring", "auto", "ar_twoshot", "ar_oneshot"] * 2):
+        for t in x + y:
+            t.fill_(-1.0)
+        torch.cuda.synchronize()
+        stream = streams[it // 2 % 2] if it % 4 else streams[0]
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(4_000_000)
+            for r in range(n):
+                x[r].fill_(float(it + r))
+        with M.group():
+            for r in range(n):
+                comms[r].all_reduce(x[r], y[r], algo=algo, stream=stream)
+        assert algo == "auto" or comms[0].last_plan()[0] == algo
+        comms[it % 2].wait(other)
+        with torch.cuda.stream(other):
+            seen = [t.clone() for t in y]
+        torch.cuda.synchronize()
+        assert all(bool((t == float(2 * it + 1)).all()) for t in seen), (it, algo, seen[0][:4].tolist())
+    for algo in ("ar_twoshot", "auto"):
+        extra = [M.Buffer(count * 4, 0) for _ in range(n)]
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(100_000_000)       # about 50 ms
+        with M.group():
+            for r in range(n):
+                comms[r].all_reduce(x[r], extra[r].tensor(torch.float32, count), algo=algo, stream=streams[0])
+        assert not streams[0].query()
+        extra[0].free()
+        assert streams[0].query()
+        extra[1].free()
+    for c in comms:
+        q = c.query()
+        assert q["async_error"] == 0 and q["device_error"] == 0
+        c.destroy()
+
+
 FUSED = r"""
 import os, threading
 import torch
