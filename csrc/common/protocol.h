@@ -157,6 +157,7 @@ struct CommInitReply {
   // events in between. `status_va`: the status block whose done_seq tells what has finished.
   uint32_t caller_streams;
   uint64_t status_va;
+  uint64_t rank_stream;                   // with caller_streams: the daemon's own stream of this rank (see DpStatus::given_up)
 };
 
 struct CommDestroyReq { Header h; uint64_t comm_handle; };
@@ -323,7 +324,14 @@ struct alignas(64) DpStatus {
   uint32_t last_ctas;
   uint32_t pad_;
   uint64_t group_closed;   // written by the client: its newest request when it last closed a group
-  uint32_t pad2_[8];
+  // Requests that name their caller's stream (kWrCallerStream) and whose call has ended without an answer.
+  // The caller may destroy the stream then, so such requests, up to number `given_up`, go to the rank's own
+  // stream instead, which the client has put behind the caller's. The client writes `given_up` and then
+  // waits until `streams_in_use` is zero; the daemon sets that around its use of callers' streams and
+  // reads `given_up` behind it: one of the two sees the other.
+  uint64_t given_up;
+  uint32_t streams_in_use;
+  uint32_t pad2_[5];
 };
 static_assert(sizeof(DpStatus) == 64, "DpStatus layout is part of the ABI");
 

@@ -686,6 +686,7 @@ void Daemon::on_comm_init(Session& s, const proto::CommInitReq& m) {
       r.comm_init_reply.fifo_slot_bytes = (uint32_t)cptr->fifo_slot_bytes;
       r.comm_init_reply.caller_streams = cptr->caller_streams ? 1u : 0u;
       r.comm_init_reply.status_va = cptr->caller_streams ? (uint64_t)cptr->ranks[0]->status : 0;
+      r.comm_init_reply.rank_stream = cptr->caller_streams ? (uint64_t)rs.stream : 0;
       r.comm_init_reply.group_defer = cptr->client_launch && cfg_.fuse_allreduce > 1 ? 1u : 0u;
       int fds[2] = {rs.dp_fd, -1};
       int nfds = 1;

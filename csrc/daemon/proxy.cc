@@ -819,6 +819,32 @@ void ProxyEngine::fill_args(Communicator& c, CollSlot& s, int rank, int slice, C
   for (int ch = 0; ch < kMaxRingChannels; ch++) a.ring_step_base[ch] = s.ring_step_base[ch];
 }
 
+namespace {
+// While this exists the callers' streams that a launch is about to use stay valid: a call that gives its
+// request up in the meantime waits for the end of it, one that has done so before has its rank's own
+// stream in place of its own (proto::DpStatus::given_up).
+struct CallerStreamsInUse {
+  Communicator& c;
+  CallerStreamsInUse(Communicator& comm, CollSlot& s, uint64_t seq) : c(comm) {
+    if (!c.caller_streams) return;
+    const int len = s.fused_kernel ? s.batch_len : 1;
+    for (int r = 0; r < c.nranks; r++) {
+      RankState& rr = *c.ranks[(size_t)r];
+      __atomic_store_n(&rr.dp_status->streams_in_use, 1u, __ATOMIC_SEQ_CST);
+      const uint64_t given_up = __atomic_load_n(&rr.dp_status->given_up, __ATOMIC_SEQ_CST);
+      for (int k = 0; k < len && given_up; k++) {
+        CollOp& op = (k == 0 ? s : c.slot(seq + (uint64_t)k)).ops[r];
+        if (op.on_caller_stream && op.user_seq <= given_up) op.caller_stream = rr.stream;
+      }
+    }
+  }
+  ~CallerStreamsInUse() {
+    if (!c.caller_streams) return;
+    for (auto& r : c.ranks) __atomic_store_n(&r->dp_status->streams_in_use, 0u, __ATOMIC_RELEASE);
+  }
+};
+}  // namespace
+
 bool ProxyEngine::launch_slices(RankState& rs, CollSlot& s, uint64_t seq) {
   Communicator& c = *rs.comm;
   Backend* be = daemon_->backend();
@@ -847,13 +873,14 @@ bool ProxyEngine::launch_slices(RankState& rs, CollSlot& s, uint64_t seq) {
       be->event_record(rs.device, rs.backend_event, rs.stream);
     return true;
   }
+  CallerStreamsInUse in_use(c, s, seq);
   void* const stream = op.on_caller_stream ? op.caller_stream : rs.stream;
+  bool ordered = false;
   while (rs.next_slice < s.nslices) {
     if (!admit_slice(c, s, rs.next_slice)) return false;
-    if (rs.next_slice == 0) {
-      if (!op.on_caller_stream) order_after_client(rs, op, stream);
-      order_after_last_launch(c, stream);
-    }
+    if (rs.next_slice == 0 && !op.on_caller_stream) order_after_client(rs, op, stream);
+    if (!ordered) order_after_last_launch(c, stream);   // as in launch_group
+    ordered = true;
     CollArgs a;
     fill_args(c, s, rs.rank, rs.next_slice, &a);
     int rc = be->launch(rs.device, op.kind, a, s.plan.dims, stream);
@@ -1022,6 +1049,7 @@ void ProxyEngine::end_group(Communicator& c, CollSlot& s, uint64_t seq, void* st
 bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
   RankState& r0 = *c.ranks[0];
   Backend* be = daemon_->backend();
+  CallerStreamsInUse in_use(c, s, seq);
   void* const stream = stream_for_group(c, s, seq);
   if (s.fused_kernel) {
     if (!admit_slice(c, s, 0)) return false;
@@ -1042,9 +1070,11 @@ bool ProxyEngine::launch_group(Communicator& c, CollSlot& s, uint64_t seq) {
     s.group_launch.store(2, std::memory_order_release);
     return true;
   }
+  bool ordered = false;
   while (r0.next_slice < s.nslices) {
     if (!admit_slice(c, s, r0.next_slice)) return false;
-    if (r0.next_slice == 0) begin_group(c, s, seq, stream);
+    if (!ordered) begin_group(c, s, seq, stream);   // again when slices had to wait: the streams may be other ones by now
+    ordered = true;
     CollArgs a;
     fill_args(c, s, 0, r0.next_slice, &a);
     int rc = be->launch(r0.device, s.ops[0].kind, a, s.plan.dims, stream);

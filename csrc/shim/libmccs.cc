@@ -16,6 +16,7 @@
 #include <poll.h>
 #include <pthread.h>
 #include <stdio.h>
+#include <sched.h>
 #include <stdlib.h>
 #include <string.h>
 #include <sys/mman.h>
@@ -23,6 +24,7 @@
 #include <time.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <map>
@@ -75,6 +77,7 @@ struct Driver {
   DRV_FN(cuMemHostUnregister);
   DRV_FN(cuMemHostGetDevicePointer);
   DRV_FN(cuCtxSynchronize);
+  DRV_FN(cuStreamSynchronize);
   bool memops = false;
 };
 Driver g_drv;
@@ -114,6 +117,7 @@ bool load_driver() {
                  sym(l, "cuMemHostUnregister", &g_drv.cuMemHostUnregister_) &&
                  sym(l, "cuMemHostGetDevicePointer_v2", &g_drv.cuMemHostGetDevicePointer_);
   sym(l, "cuCtxSynchronize", &g_drv.cuCtxSynchronize_);
+  sym(l, "cuStreamSynchronize", &g_drv.cuStreamSynchronize_);
   if (g_drv.ok && g_drv.cuInit_(0) != CUDA_SUCCESS) g_drv.ok = false;
   return g_drv.ok;
 }
@@ -234,6 +238,7 @@ struct mccsComm {
   // submitted that way has finished.
   bool caller_streams = false;
   const uint64_t* done_seq = nullptr;
+  mccsStream_t rank_stream = nullptr;   // the daemon's stream of this rank, for requests that are given up
   uint64_t last_ticket = 0;
   uint32_t last_ticket_variant = 0;   // the kernel that raises done_seq to it
   bool deferred_wait = false;         // collectives do not queue "wait done"; mccsCommWait does
@@ -697,6 +702,24 @@ mccsResult_t wait_completion(mccsComm* comm, proto::WorkCompletion* wc) {
   if (wc->ticket) { comm->last_ticket = wc->ticket; comm->last_ticket_variant = wc->variant; }
   if (wc->status != 0 && comm->sticky_error == 0) comm->sticky_error = wc->status;
   return (mccsResult_t)wc->status;
+}
+
+// A call on `streams` ends although requests of it are still unanswered: from here on the daemon keeps off
+// the streams, and launches what it still gets to on the rank's own stream, behind what the caller has
+// queued so far (see proto::DpStatus::given_up).
+void give_up_streams(mccsComm* comm, const std::vector<mccsStream_t>& streams) {
+  if (!comm->caller_streams || !comm->dp_status || comm->outstanding == 0) return;
+  CtxScope scope(comm->device);
+  CUevent mark = nullptr;
+  if (!scope.ok || g_drv.cuEventCreate_(&mark, CU_EVENT_DISABLE_TIMING) != CUDA_SUCCESS) mark = nullptr;
+  for (mccsStream_t s : streams) {
+    const bool behind = mark && g_drv.cuEventRecord_(mark, (CUstream)s) == CUDA_SUCCESS &&
+                        g_drv.cuStreamWaitEvent_((CUstream)comm->rank_stream, mark, 0) == CUDA_SUCCESS;
+    if (!behind && scope.ok && g_drv.cuStreamSynchronize_) g_drv.cuStreamSynchronize_((CUstream)s);
+  }
+  if (mark) g_drv.cuEventDestroy_(mark);
+  __atomic_store_n(&comm->dp_status->given_up, comm->next_user_seq - 1, __ATOMIC_SEQ_CST);
+  while (__atomic_load_n(&comm->dp_status->streams_in_use, __ATOMIC_SEQ_CST)) sched_yield();
 }
 
 mccsResult_t finish_on_stream(mccsComm* comm, mccsStream_t stream) {
@@ -1172,6 +1195,19 @@ mccsResult_t submit_client_launch(mccsComm* comm, proto::WorkRequest& wr, mccsSt
   return run_planned(comm, wr.user_seq, plan, stream);
 }
 
+// The same for the communicators of a group.
+void give_up_group(const std::vector<GroupItem>& items) {
+  std::vector<mccsComm*> done;
+  for (const GroupItem& it : items) {
+    if (std::find(done.begin(), done.end(), it.comm) != done.end()) continue;
+    done.push_back(it.comm);
+    std::vector<mccsStream_t> streams;
+    for (const GroupItem& same : items)
+      if (same.comm == it.comm && same.ordered && std::find(streams.begin(), streams.end(), same.stream) == streams.end()) streams.push_back(same.stream);
+    give_up_streams(it.comm, streams);
+  }
+}
+
 mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, void* recv, uint64_t send_bytes,
                     uint64_t recv_bytes, mccsStream_t stream) {
   if (!comm) return mccsInvalidArgument;
@@ -1234,7 +1270,10 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
   mccsResult_t r = mccsSuccess;
   while (comm->outstanding > 0) {
     mccsResult_t one = wait_completion(comm, &wc);
-    if (one == mccsTimeout || one == mccsNotConnected) return one;
+    if (one == mccsTimeout || one == mccsNotConnected) {
+      if (on_caller_stream) give_up_streams(comm, {stream});
+      return one;
+    }
     if (one != mccsSuccess) r = one;
   }
   if (r != mccsSuccess) return r;
@@ -1478,7 +1517,10 @@ mccsResult_t mccsCommInitRank(mccsComm_t* comm, uint32_t unique_id, int rank, in
   c->group_defer = c->client_launch && m.comm_init_reply.group_defer != 0;
   c->fifo_slot_bytes = m.comm_init_reply.fifo_slot_bytes;
   c->caller_streams = g_ctx.same_process && m.comm_init_reply.caller_streams != 0 && m.comm_init_reply.status_va != 0 && g_drv.memops;
-  if (c->caller_streams) c->done_seq = &((const StatusBlock*)m.comm_init_reply.status_va)->done_seq;
+  if (c->caller_streams) {
+    c->done_seq = &((const StatusBlock*)m.comm_init_reply.status_va)->done_seq;
+    c->rank_stream = (mccsStream_t)m.comm_init_reply.rank_stream;
+  }
   if (g_ctx.backend == proto::kBackendHost && m.comm_init_reply.sync_size && fds.size() > 1) {
     const size_t bytes = m.comm_init_reply.sync_size;
     void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_SHARED, fds[1], 0);
@@ -1599,6 +1641,12 @@ mccsResult_t mccsCommFlush(mccsComm_t comm) {
 mccsResult_t mccsCommDestroy(mccsComm_t comm) {
   if (!comm) return mccsSuccess;
   if (g_ctx.connected) mccsCommFlush(comm);   // every posted request has been taken by the daemon
+  if (comm->outstanding) {      // the flush ran out of time inside an open group
+    std::vector<GroupItem> mine;
+    for (const GroupItem& it : g_group_items)
+      if (it.comm == comm) mine.push_back(it);
+    give_up_group(mine);
+  }
   // A handle destroyed inside an open group must not be looked at again when the group ends.
   for (size_t i = g_group_items.size(); i-- > 0;)
     if (g_group_items[i].comm == comm) g_group_items.erase(g_group_items.begin() + (long)i);
@@ -1821,7 +1869,10 @@ mccsResult_t mccsGroupEnd(void) {
     proto::WorkCompletion wc;
     while (it.comm->outstanding > 0) {
       mccsResult_t r = wait_completion(it.comm, &wc);
-      if (r == mccsTimeout || r == mccsNotConnected) return r;
+      if (r == mccsTimeout || r == mccsNotConnected) {
+        give_up_group(items);
+        return r;
+      }
       if (r != mccsSuccess) result = r;
     }
   }

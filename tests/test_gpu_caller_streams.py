@@ -215,3 +215,110 @@ def test_streams_destroyed_while_their_collective_waits(service, n):
     print(f"{len(handles) - len(set(handles))} of {len(handles)} handles were given out again")
     for c in comms:
         c.destroy()
+
+
+TIMED_OUT = r"""
+import ctypes, os, threading, time
+import torch
+import mccs_b200 as M
+
+torch.cuda.set_device(0)
+M.init(M.daemon.start_embedded(prefix=f"/tmp/mccs-given-up-{os.getpid()}", listen_port=-1))
+lib, count = ctypes.CDLL("libcuda.so.1"), 1 << 20
+
+def create():
+    s = ctypes.c_void_p()
+    assert lib.cuStreamCreate(ctypes.byref(s), 1) == 0
+    return s, torch.cuda.ExternalStream(s.value)
+
+def timed_out(call):
+    try:
+        call()
+    except M.MccsError as e:
+        assert e.code == -6, e
+        return
+    raise AssertionError("the call came back")
+
+def communicators(cid, n):
+    comms = [None] * n
+    ts = [threading.Thread(target=lambda r=r: comms.__setitem__(r, M.Communicator(cid, r, n, device=0))) for r in range(n)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    return comms
+
+def pause(cid, on):
+    assert M.daemon.embedded_admin({"cmd": "pause" if on else "resume", "communicator_id": cid})["status"] == "ok"
+
+other = torch.cuda.Stream()
+for cid, n, grouped in ((51, 2, False), (52, 2, True), (53, 1, False), (54, 1, True)):
+    comms = communicators(cid, n)
+    bufs = [M.Buffer(count * 4, 0) for _ in range(2 * n)]
+    x, y = ([b.tensor(torch.float32, count) for b in bufs[i::2]] for i in range(2))
+    for t in x:
+        t.fill_(1.0)
+    with M.group():                                    # loads the kernel (which waits for a busy GPU)
+        for r in range(n):
+            comms[r].all_reduce(x[r], y[r])
+    for it in range(3):
+        for t in y:
+            t.fill_(-1.0)
+        torch.cuda.synchronize()
+        raw, stream = create()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(1_500_000_000)           # outlasts the call's patience: the input exists only after it
+            x[0].fill_(float(it + 1))
+        def first():
+            if grouped:
+                with M.group():
+                    comms[0].all_reduce(x[0], y[0], stream=stream)
+            else:
+                comms[0].all_reduce(x[0], y[0], stream=stream)
+        if n == 1:
+            pause(cid, True)
+        timed_out(first)                               # no peer (or a paused communicator)
+        assert lib.cuStreamDestroy_v2(raw) == 0        # the caller is done with its stream
+        raw2, stream2 = create()
+        if n == 1:
+            pause(cid, False)
+        else:
+            with torch.cuda.stream(stream2):
+                x[1].fill_(10.0)
+            comms[1].all_reduce(x[1], y[1], stream=stream2)
+            with torch.cuda.stream(stream2):
+                seen = y[1].clone()
+        comms[0].flush()                               # the request was carried out all the same
+        comms[0].wait(other)
+        with torch.cuda.stream(other):
+            mine = y[0].clone()
+        torch.cuda.synchronize()
+        want = float(it + 1) + (10.0 if n == 2 else 0.0)
+        assert bool((mine == want).all()), (cid, it, mine[:4].tolist(), want)
+        if n == 2:
+            assert bool((seen == want).all()), (cid, it, seen[:4].tolist(), want)
+        assert lib.cuStreamDestroy_v2(raw2) == 0
+    # and the communicator goes on as before
+    for t in x:
+        t.fill_(1.0)
+    with M.group():
+        for r in range(n):
+            comms[r].all_reduce(x[r], y[r])
+    assert all(bool((t == float(n)).all()) for t in y)
+    for c in comms:
+        c.destroy()
+M.finalize()
+M.daemon.stop_embedded()
+print("OK")
+"""
+
+
+def test_a_call_that_timed_out_gives_its_stream_back():
+    """A call that ends without its answer leaves its request behind, but not the caller's stream: the stream can be
+    destroyed, and the collective still runs behind what had been queued on it when the peers arrive."""
+    import os
+    import subprocess
+    import sys
+
+    from helpers import REPO
+    p = subprocess.run([sys.executable, "-c", TIMED_OUT], env=dict(os.environ, PYTHONPATH=REPO, MCCS_WC_TIMEOUT_MS="300"),
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and p.stdout.strip().endswith("OK"), p.stdout[-2000:] + p.stderr[-3000:]
