@@ -78,6 +78,7 @@ struct Driver {
   DRV_FN(cuMemHostGetDevicePointer);
   DRV_FN(cuCtxSynchronize);
   DRV_FN(cuStreamSynchronize);
+  DRV_FN(cuStreamIsCapturing);
   bool memops = false;
 };
 Driver g_drv;
@@ -118,6 +119,7 @@ bool load_driver() {
                  sym(l, "cuMemHostGetDevicePointer_v2", &g_drv.cuMemHostGetDevicePointer_);
   sym(l, "cuCtxSynchronize", &g_drv.cuCtxSynchronize_);
   sym(l, "cuStreamSynchronize", &g_drv.cuStreamSynchronize_);
+  sym(l, "cuStreamIsCapturing", &g_drv.cuStreamIsCapturing_);
   if (g_drv.ok && g_drv.cuInit_(0) != CUDA_SUCCESS) g_drv.ok = false;
   return g_drv.ok;
 }
@@ -1215,6 +1217,16 @@ mccsResult_t submit(mccsComm* comm, proto::WorkRequest& wr, const void* send, vo
   // (A deferred wait keeps the collective off the caller's stream; the per-thread default stream
   // is another one in the daemon's thread.)
   const bool on_caller_stream = comm->caller_streams && !comm->deferred_wait && stream != (mccsStream_t)CU_STREAM_PER_THREAD;
+  if (on_caller_stream && g_drv.cuStreamIsCapturing_) {
+    // A kernel launched on a stream under capture only becomes part of the graph: its completion word, which
+    // other streams and the daemon wait for, would not come.
+    CUstreamCaptureStatus st = CU_STREAM_CAPTURE_STATUS_NONE;
+    const CUresult r = g_drv.cuStreamIsCapturing_((CUstream)stream, &st);
+    if (r == CUDA_ERROR_STREAM_CAPTURE_IMPLICIT || (r == CUDA_SUCCESS && st != CU_STREAM_CAPTURE_STATUS_NONE)) {
+      LOG_ERROR("a collective on a stream under capture");
+      return mccsUnsupported;
+    }
+  }
   {
     std::unique_lock<std::mutex> g(g_ctx.mu);
     if (!g_ctx.connected) return mccsNotConnected;

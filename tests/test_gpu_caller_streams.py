@@ -322,3 +322,37 @@ def test_a_call_that_timed_out_gives_its_stream_back():
     p = subprocess.run([sys.executable, "-c", TIMED_OUT], env=dict(os.environ, PYTHONPATH=REPO, MCCS_WC_TIMEOUT_MS="300"),
                        capture_output=True, text=True, timeout=300)
     assert p.returncode == 0 and p.stdout.strip().endswith("OK"), p.stdout[-2000:] + p.stderr[-3000:]
+
+
+@pytest.mark.parametrize("n", [1, 2])
+def test_a_named_stream_under_capture_is_refused(service, n):
+    """The refusal of graph capture looks at the stream the collective is given, not only at the current one."""
+    M = service
+    torch.cuda.set_device(0)
+    cid, comms = fresh_comm_id(), [None] * n
+    run_ranks(n, lambda r: comms.__setitem__(r, M.Communicator(cid, r, n, device=0)))
+    bufs = [M.Buffer(4096, 0) for _ in range(n)]
+    x = [b.tensor(torch.float32) for b in bufs]
+    for t in x:
+        t.fill_(1.0)
+    scratch = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode="relaxed")
+        scratch.add_(1.0)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for c, t in zip(comms, x):
+                with pytest.raises(M.MccsError, match="-9"):
+                    c.all_reduce(t, stream=stream)
+        graph.capture_end()
+    with M.group():
+        for c, t in zip(comms, x):
+            c.all_reduce(t)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(bool((t == float(n)).all()) for t in x) and bool((scratch == 1.0).all())
+    for c in comms:
+        q = c.query()
+        assert q["async_error"] == 0 and q["device_error"] == 0
+        c.destroy()
