@@ -30,10 +30,11 @@ APPS := allreduce_bench allgather_bench allreduce_proto allgather_proto reducesc
 APP_BINS := $(addprefix $(OUT)/,$(APPS))
 
 # CPython extension of the collective calls, built for the interpreter that runs the package and
-# the torch installed there (found without importing it).
+# the torch installed there (found without importing it), with its CUDA library where it has one.
 PYTHON  ?= python3
 PYINC    = $(shell $(PYTHON) -c "import sysconfig; print(sysconfig.get_paths()['include'])")
-TORCHDIR = $(shell $(PYTHON) -c "import importlib.util, os; print(os.path.dirname(importlib.util.find_spec('torch').origin))")
+TORCHDIR := $(shell $(PYTHON) -c "import importlib.util, os; print(os.path.dirname(importlib.util.find_spec('torch').origin))")
+TORCHCUDA = $(wildcard $(TORCHDIR)/lib/libc10_cuda.so)
 
 all: $(OUT)/_calls.so $(OUT)/libmccs_daemon.so $(OUT)/libmccs.so $(OUT)/libmccs_kernels.so $(OUT)/mccsd $(OUT)/libmccs_preload.so $(APP_BINS) $(OUT)/host_tests
 
@@ -80,10 +81,10 @@ $(OUT)/libmccs.so: $(SHIM_OBJS) $(EMU_OBJ) csrc/exports.map
 	@mkdir -p $(OUT)
 	$(CXX) -shared -Wl,--version-script=csrc/exports.map -o $@ $(SHIM_OBJS) $(EMU_OBJ) $(LDLIBS)
 
-$(OUT)/_calls.so: csrc/python/calls.cc csrc/include/mccs.h csrc/include/mccs_noalloc.h
+$(OUT)/_calls.so: csrc/python/calls.cc csrc/include/mccs.h csrc/include/mccs_noalloc.h $(wildcard $(TORCHDIR)/version.py)
 	@mkdir -p $(OUT)
-	$(CXX) $(CXXFLAGS) -g0 -fvisibility=hidden -Wl,--exclude-libs,ALL -Wno-missing-field-initializers -I$(PYINC) -isystem $(TORCHDIR)/include -shared -o $@ $< \
-	    -L$(TORCHDIR)/lib -ltorch_python -ltorch -ltorch_cpu -lc10_cuda -lc10 -ldl
+	$(CXX) $(CXXFLAGS) -g0 -fvisibility=hidden -Wl,--exclude-libs,ALL -Wno-missing-field-initializers -I$(PYINC) -isystem $(TORCHDIR)/include $(if $(TORCHCUDA),-DMCCS_TORCH_CUDA) -shared -o $@ $< \
+	    -L$(TORCHDIR)/lib -ltorch_python -ltorch -ltorch_cpu $(if $(TORCHCUDA),-lc10_cuda) -lc10 -ldl
 
 $(OUT)/libmccs_preload.so: $(OBJ)/shim/preload.o $(OUT)/libmccs.so
 	$(CXX) -shared -Wl,--version-script=csrc/exports_preload.map -o $@ $(OBJ)/shim/preload.o -L$(OUT) -lmccs -Wl,-rpath,'$$ORIGIN' $(LDLIBS)

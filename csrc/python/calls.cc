@@ -16,13 +16,16 @@
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/InferenceMode.h>
+#ifdef MCCS_TORCH_CUDA
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#endif
 #include <cuda.h>
 #include <dlfcn.h>
 #include <stdint.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/headeronly/version.h>
 
 #include "../include/mccs.h"
 #include "../include/mccs_noalloc.h"
@@ -60,6 +63,16 @@ struct Calls {
 };
 
 const at::Tensor* tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+// torch's current stream on a device and its current device. A torch without CUDA has neither (and no CUDA
+// tensors): the daemon's host backend needs none, a GPU's wants the stream named.
+#ifdef MCCS_TORCH_CUDA
+uint64_t current_stream(int device) { return (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
+int current_device() { return (int)c10::cuda::current_device(); }
+#else
+uint64_t current_stream(int) { throw std::runtime_error("this torch is built without CUDA: a collective on a GPU needs stream="); }
+int current_device() { return -1; }
+#endif
 
 // mccsDataType_t of a tensor, if there is one.
 bool known_type(const at::Tensor& t, int* out) {
@@ -153,7 +166,11 @@ PyObject* raise(int code, const char* what) {
 bool resolve_stream(Calls* self, PyObject* stream, uint64_t* out) {
   *out = 0;
   if (self->cuda) {
-    const uint64_t current = (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
+#ifdef MCCS_TORCH_CUDA
+    const uint64_t current = current_stream(self->device);
+#else
+    const uint64_t current = stream && stream != Py_None ? 0 : current_stream(self->device);
+#endif
     bool capturing = false, known = false;
     CUdevice now = -1;
     if (g_is_capturing && g_ctx_device && g_ctx_device(&now) == CUDA_SUCCESS && (int)now == self->device) {
@@ -320,7 +337,7 @@ PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   if (service ? !known_type(*in, &dtype) : autograd_takes_part(*in, *out)) Py_RETURN_FALSE;
   // The tensors belong to the current stream's order, whichever stream the collective is given: the staged
   // form copies there.
-  if (!service && stream != (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()) Py_RETURN_FALSE;
+  if (!service && stream != current_stream(self->device)) Py_RETURN_FALSE;
   mccsResult_t rc;
   const mccsComm_t comm = self->comm;
   Py_BEGIN_ALLOW_THREADS
@@ -433,10 +450,10 @@ PyObject* local_all_reduce(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Py_DECREF(seq[1]);
   if (bad) { PyErr_SetString(PyExc_ValueError, bad); return nullptr; }
   // (The runtime's device: a thread that has not used CUDA yet has one, but no context of the driver's.)
-  if ((int)c10::cuda::current_device() != device) Py_RETURN_NONE;
+  if (current_device() != device) Py_RETURN_NONE;
   uint64_t stream = 0;
   if (args[3] == Py_None) {
-    stream = (uint64_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+    stream = current_stream(device);
   } else {
     PyObject* h = PyObject_GetAttr(args[3], s_cuda_stream);
     const bool ok = h && to_u64(h, &stream);
@@ -500,5 +517,6 @@ PyMODINIT_FUNC PyInit__calls(void) {
   PyObject* m = PyModule_Create(&module_def);
   if (!m) return nullptr;
   PyModule_AddObject(m, "CommCalls", Py_NewRef((PyObject*)&calls_type));
+  PyModule_AddStringConstant(m, "built_for", TORCH_VERSION);   // it reads tensors through this version's C++ interface
   return m;
 }

@@ -149,13 +149,19 @@ def calls():
         import importlib.machinery
         import importlib.util
 
-        import torch  # noqa: F401  (the extension links against its libraries)
+        import torch   # the extension links against its libraries
         path = os.path.join(NATIVE_DIR, "_calls.so")
         if not os.path.exists(path):
             raise ImportError(f"{path} is missing: build the native code with `make -j` at the repository root")
         loader = importlib.machinery.ExtensionFileLoader("mccs_b200._calls", path)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("mccs_b200._calls", loader))
-        loader.exec_module(mod)
+        rebuild = "rebuild it for this torch with `make -j` at the repository root"
+        try:
+            loader.exec_module(mod)
+        except ImportError as e:
+            raise ImportError(f"{path} does not load next to torch {torch.__version__} ({e}): {rebuild}") from e
+        if mod.built_for != torch.__version__.split("+")[0]:
+            raise ImportError(f"{path} was built for torch {mod.built_for}, not {torch.__version__}: {rebuild}")
         bind_calls(mod)
         _calls = mod
     return _calls

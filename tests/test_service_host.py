@@ -341,3 +341,54 @@ def test_collectives_refuse_cuda_graph_capture(service, monkeypatch):
         c = M.Communicator(cid, 0, 1, device=0)
         c.all_reduce(buf.tensor(torch.float32, 16))
         c.destroy()
+
+
+def test_native_calls_are_checked_against_the_installed_torch(monkeypatch):
+    """The extension reads tensors through the C++ interface of the torch it was built for."""
+    from mccs_b200 import _lib
+    assert _lib.calls().built_for == torch.__version__.split("+")[0]
+    monkeypatch.setattr(_lib, "_calls", None)
+    monkeypatch.setattr(torch, "__version__", "1.0.0+cpu")
+    with pytest.raises(ImportError, match="rebuild"):
+        _lib.calls()
+
+
+CPU_TORCH = r"""
+import sys, threading, torch
+from mccs_b200 import _lib
+_lib.NATIVE_DIR = sys.argv[1]
+import mccs_b200 as M
+M.init(M.daemon.start_embedded(prefix=sys.argv[1] + "/run", listen_port=-1, force_host=True, host_devices=2))
+out = [None, None]
+def rank(r):
+    buf = M.Buffer(4096, r)
+    t = buf.tensor(torch.float32)
+    t.fill_(r + 1.0)
+    c = M.Communicator(9, r, 2, device=r)
+    c.all_reduce(t)
+    from mccs_b200 import ops
+    u = ops.all_reduce(c, torch.full((10,), r + 2.0))
+    out[r] = (float(t[0]), float(u[0]))
+    c.destroy()
+ts = [threading.Thread(target=rank, args=(r,)) for r in range(2)]
+[t.start() for t in ts]; [t.join() for t in ts]
+M.finalize(); M.daemon.stop_embedded()
+assert out == [(3.0, 5.0)] * 2, out
+print("OK")
+"""
+
+
+def test_native_calls_build_for_a_torch_without_cuda(tmp_path):
+    """Without torch's CUDA library the extension is built without it, and the host backend works as ever."""
+    import shutil
+    import subprocess
+
+    from helpers import NATIVE, REPO, run_python
+    res = subprocess.run(["make", f"OUT={tmp_path}", "TORCHCUDA=", f"{tmp_path}/_calls.so"], cwd=REPO, capture_output=True, text=True, timeout=600)
+    assert res.returncode == 0, res.stderr[-3000:]
+    needed = subprocess.run(["readelf", "-d", f"{tmp_path}/_calls.so"], capture_output=True, text=True).stdout
+    assert "libtorch_python.so" in needed and "cuda" not in needed, needed
+    for f in ("libmccs.so", "libmccs_daemon.so", "libmccs_kernels.so"):
+        shutil.copy(f"{NATIVE}/{f}", tmp_path)
+    p = run_python(f"import sys; sys.argv = ['-', {str(tmp_path)!r}]\n" + CPU_TORCH)
+    assert p.returncode == 0 and p.stdout.strip().endswith("OK"), p.stdout + p.stderr[-3000:]
