@@ -5,8 +5,10 @@
 // rendezvous slot for that collective, (3) once every rank has posted, one proxy
 // plans the collective for all ranks (variant, CTAs, slices, barrier epochs, NVLS
 // mappings), (4) asks the QoS arbiter for admission, slice by slice, (5) launches
-// the kernel on the rank's backend stream between the client's "submitted" event
-// and the backend's "done" event, and (6) completes the request.
+// the kernel, and (6) completes the request. (5) takes one of three forms: on the
+// backend's stream between the client's "submitted" mark and the backend's "done" mark
+// (events or semaphores); on the caller's own stream, for clients inside the daemon's process whose
+// ranks are on one GPU; or not at all, when the client library launches from the plan it is handed.
 //
 // Reference counterparts: check_daemon_command / schedule_all_reduce /
 // launch_scheduled_and_record (src/mccs/src/proxy/engine.rs:926-1066,1170-1275) and

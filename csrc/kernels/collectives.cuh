@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(kMaxThreads) local_copy_kernel(const __grid_co
   const uint64_t bytes = a.count;  // the launcher converts elements to bytes
   if (in != out) {
     uint64_t done = 0;
-    if ((((uint64_t)in | (uint64_t)out) & 15u) == 0) {   // (elsewhere local_copy_ragged_kernel is the faster one)
+    if ((((uint64_t)in | (uint64_t)out) & 15u) == 0) {   // (the GPU launcher has local_copy_ragged_kernel for the others, the emulator has not)
       const uint64_t nv = bytes / 16;
       const uint64_t tile = (uint64_t)blockDim.x * kCopyUnroll;
       const Raw<16>* src = (const Raw<16>*)in;

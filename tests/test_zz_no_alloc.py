@@ -3,10 +3,9 @@ its exported C symbol, against the service's regular AllReduce on the same input
 
 Who needs the entry point: callers that may not allocate when they reduce — inside a
 frozen or exhausted memory pool, in callbacks and latency-critical sections that must
-not enter the CUDA allocator. It keeps its synchronisation scratch in a static device
-array, so consecutive calls share state; two calls in a row check that the second one
-starts from a clean slate. Further cases: free device memory does not move across calls,
-the kernels' status words can be read back, and the aliasing rules. This file is collected last on purpose: a failure here
+not enter the CUDA allocator. Calls share no state; two calls in a row check that the second
+one does not see the first. Further cases: free device memory does not move across calls,
+the kernels' status words can be read back, the aliasing rules, what Prepare loads. This file is collected last on purpose: a failure here
 leaves every other test already run."""
 import ctypes
 
@@ -58,7 +57,7 @@ def test_no_alloc_entry_matches_service(service, dtype, n, count):
     torch.cuda.set_device(0)
     stream = torch.cuda.current_stream()
     tol = 1e-5 if dtype == torch.float32 else 1.6e-2
-    for call in range(2):                      # two calls in a row share the static scratch
+    for call in range(2):
         g = torch.Generator().manual_seed(50 + call)
         inputs = [((torch.rand(count, generator=g) * 2 - 1).to(dtype)).cuda() for _ in range(n)]
         outputs = [torch.empty_like(x) for x in inputs]
@@ -137,7 +136,7 @@ def test_no_alloc_entry_rejects_what_it_cannot_do(service):
     x = torch.zeros(16, device="cuda")
     one = (ctypes.c_void_p * 1)(x.data_ptr())
     many = (ctypes.c_void_p * 9)(*([x.data_ptr()] * 9))
-    assert fn(many, many, 9, 16, 7, None) != 0        # more buffers than the scratch has slots for
+    assert fn(many, many, 9, 16, 7, None) != 0        # more buffers than the entry point takes
     assert fn(one, one, 1, 16, 2, None) != 0          # int32 is not offered
     assert fn(one, one, 0, 16, 7, None) != 0
     assert fn(one, one, 1, 16, 7, None) == 0          # single buffer in place: nothing to do, still valid

@@ -3,7 +3,7 @@
 staging arena (copy in, collective in place, copy out, all on the caller's stream), tensors
 in service memory are used where they are. Two client processes of a stand-alone daemon; on
 a machine with one GPU both sit on cuda:0 (the daemon then runs each collective as one
-cooperative launch), with two or more each has its own.
+launch for both ranks), with two or more each has its own.
 
 The reference has no framework layer; parity is with what the same calls give on the
 ``nccl`` backend: the values asserted below.
