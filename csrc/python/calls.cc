@@ -315,7 +315,7 @@ bool autograd_takes_part(const at::Tensor& in, const at::Tensor& out) {
 // self_copy(send, recv, stream) -> bool. Any collective of a communicator of one rank whose tensors
 // are plain memory of its GPU: one copy kernel on them where they are. False when that does not apply
 // (more ranks, other devices, other layouts, differing types, values that are not the bytes, ranges that
-// overlap in part) and the caller has to stage.
+// overlap in part, another stream than the current one) and the caller has to stage.
 PyObject* self_copy(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
   Calls* self = (Calls*)self_;
   if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "self_copy(send, recv, stream)"); return nullptr; }
